@@ -132,7 +132,6 @@ class ModelT final : public Model {
     CK(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
     if (prepare_acoustic_column<R>(g_.nz) || prepare_kessler<R>(g_.nz) || prepare_sfc<R>(g_.nz))
       return fail("nz too large for the column kernels' shared memory");
-    tma_ok_ = tensor_map_encoder() && prepare_acoustic_column_tma<R>(g_.nz) == 0;
     fused_ok_ = prepare_acoustic_fused<R>(g_.nz) == 0;
     pipe_ok_ = tensor_map_encoder() && prepare_acoustic_pipe<R>(g_.nz) == 0;
     uvp_ok_ = tensor_map_encoder() && prepare_acoustic_uv_pipe<R>() == 0;
@@ -856,7 +855,7 @@ class ModelT final : public Model {
     std::string name = prop.name;
     for (char& ch : name)
       if (ch == ' ') ch = '_';
-    k << "v8|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
+    k << "v9|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
       << dp_.moisture << "pd" << dp_.pd_moist << "b" << bdy_on_ << "d" << (dp_.diff_K > 0) << "x"
       << (pcr_allowed() ? 0 : 1);
     return k.str();
@@ -900,8 +899,8 @@ class ModelT final : public Model {
   }
 
   // WFE_COLUMN_VARIANT=<n> forces the acoustic variant (0..5 column tile
-  // shapes, 6 the TMA-staged column, 7..9 the fused substep kernel in three
-  // tile shapes, 10..12 the chunked column kernel, 13..15 the persistent
+  // shapes, 6 the first of them again -- the number of a kernel that is
+  // gone --, 7..9 the fused substep kernel in three tile shapes, 10..12 the chunked column kernel, 13..15 the persistent
   // pipelined column kernel, 16..18 the parallel-solve column kernel and
   // 19..22 its pipelined form, both equal to the others up to rounding),
   // WFE_UV_VARIANT=<n> the forward u, v kernel (0
@@ -916,9 +915,8 @@ class ModelT final : public Model {
     const char* cv = std::getenv("WFE_COLUMN_VARIANT");
     if (first && cv && *cv) {
       const int v = std::atoi(cv);
-      if (v >= 0 && (v < acoustic_column_shapes() || (v == acoustic_column_shapes() && tma_ok_) ||
-                     fused_usable(v) || chunked_usable(v) || pipe_usable(v) || pcr_usable(v) ||
-                     pipe_pcr_usable(v)))
+      if (v >= 0 && (v <= acoustic_column_shapes() || fused_usable(v) || chunked_usable(v) || pipe_usable(v) ||
+                     pcr_usable(v) || pipe_pcr_usable(v)))
         tune_.column_cx = v;
     }
     const char* uvv = std::getenv("WFE_UV_VARIANT");
@@ -979,12 +977,11 @@ class ModelT final : public Model {
     }
     tune_.uv_variant = cached.uv_variant;
     best = 1e30f;
-    // tile shapes, the TMA-staged column, the fused substep kernels
+    // tile shapes, the fused substep kernels (number 6 stays free)
     const int nvar = acoustic_column_shapes() + 1 + acoustic_fused_shapes() + acoustic_chunked_shapes() +
                      acoustic_pipe_shapes() + acoustic_pcr_shapes() + acoustic_pipe_pcr_shapes();
     for (int cx = 0; cx < nvar; ++cx) {
-      if (cx == acoustic_column_shapes() && !tma_ok_) continue;
-      if (cx > acoustic_column_shapes() && !fused_usable(cx) && !chunked_usable(cx) &&
+      if (cx >= acoustic_column_shapes() && !fused_usable(cx) && !chunked_usable(cx) &&
           !pipe_usable(cx) && !pcr_usable(cx) && !pipe_pcr_usable(cx))
         continue;
       // the parallel-solve variants agree with the others to rounding only:
@@ -1180,10 +1177,6 @@ class ModelT final : public Model {
       PipeColParams<R> pp;
       if (pipe_params(a, f, &pp)) return 1;
       launch("acoustic_column", [&] { rc = launch_acoustic_column_pipe<R>(pp, f, st_); });
-    } else if (tma_ok_ && v == acoustic_column_shapes()) {
-      TmaColParams<R> tp;
-      if (tma_params(a, &tp)) return 1;
-      launch("acoustic_column", [&] { rc = launch_acoustic_column_tma<R>(tp, st_); });
     } else {
       launch("acoustic_column",
              [&] { rc = launch_acoustic_column<R>(a, v < acoustic_column_shapes() ? v : 0, st_); });
@@ -1263,31 +1256,6 @@ class ModelT final : public Model {
     return 0;
   }
 
-  // tensor map of a pitched field for box f of the TMA column kernel (cached)
-  const CUtensorMap* tmap(const R* ptr, int f) {
-    int bx, by;
-    tma_col_box(f, &bx, &by);
-    const auto key = std::make_pair(static_cast<const void*>(ptr), bx * 16 + by);
-    auto it = tmaps_.find(key);
-    if (it != tmaps_.end()) return &it->second;
-    CUtensorMap m;
-    std::memset(&m, 0, sizeof(m));
-    const cuuint64_t dims[3] = {(cuuint64_t)L_.px, (cuuint64_t)L_.py, (cuuint64_t)L_.pz};
-    const cuuint64_t strides[2] = {(cuuint64_t)L_.px * sizeof(R), (cuuint64_t)L_.plane() * sizeof(R)};
-    const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)(g_.nz + 2)};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = tensor_map_encoder()(
-        &m, sizeof(R) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-        const_cast<R*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-      fail("cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
-      return nullptr;
-    }
-    return &(tmaps_[key] = m);
-  }
-
   bool tend_tma_usable() const { return tend_tma_ok_ && !(dp_.moisture && dp_.pd_moist); }
 
   // tensor map of a pitched field with box (bx, by, bz) (cached per pointer and box)
@@ -1329,24 +1297,6 @@ class ModelT final : public Model {
       const CUtensorMap* x = tmap3(q[f], kTtX + 8, kTtY + 6, kTtZ + 6);
       if (!x) return 1;
       tp->q[f] = *x;
-    }
-    return 0;
-  }
-
-  int tma_params(const AcouArgs<R>& a, TmaColParams<R>* tp) {
-    std::memset(static_cast<void*>(tp), 0, sizeof(*tp));
-    tp->a = a;
-    tp->err = tma_err_;
-    tp->has_tpi = a.tpi != nullptr;
-    const R* src[TC_N] = {a.u_out,  a.co.rtjx, a.v_out, a.co.rtjy, a.w_in,   a.pi_cur,
-                          a.th_in,  a.tw,      a.tth,   a.tpi,     a.co.aw,  a.co.kt3,
-                          a.b.thbw, a.b.dthbdz, a.qv,   a.qc,      a.qr,     a.b.qvb};
-    for (int f = 0; f < TC_N; ++f) {
-      if (f == TC_TPI && !a.tpi) continue;
-      if (f >= TC_QV && !a.p.moisture) continue;
-      const CUtensorMap* m = tmap(src[f], f);
-      if (!m) return 1;
-      tp->map[f] = *m;
     }
     return 0;
   }
@@ -1692,7 +1642,6 @@ class ModelT final : public Model {
   bool graphs_valid_ = false;
   long gen_ = 0;  // changes whenever buffer roles or physics switches change
   std::vector<Rec>* rec_ = nullptr;  // record mode when set
-  bool tma_ok_ = false;              // TMA column variant usable
   bool fused_ok_ = false;            // fused substep kernels prepared
   bool pipe_ok_ = false;             // pipelined column kernels prepared
   bool uvp_ok_ = false;              // pipelined u, v kernel prepared
