@@ -120,11 +120,11 @@ DRY_KERNEL_FIELDS = dict(KERNEL_FIELDS, acoustic_column=16, acoustic_uv=10, tend
 STEP_FIELDS = 3 * 19 + 10 * 26 + 12
 DRY_STEP_FIELDS = 3 * 10 + 10 * 22
 # With the column coefficients in per-level tables (a horizontally uniform
-# set-up and a pipelined column kernel, variants 13-15 and 19-22) a column
+# set-up and a register-held or pipelined column kernel, 10-15 and 19-22) a column
 # launch reads none of theta_b^w, dtheta_b/dz, rtjx, rtjy, kt3, aw, qv_b per
 # cell: 7 fields fewer (6 dry).
 TABLE_FIELDS, DRY_TABLE_FIELDS = 7, 6
-PIPE_VARIANTS = set(range(13, 16)) | set(range(19, 23))
+PIPE_VARIANTS = set(range(10, 16)) | set(range(19, 23))
 # With the base state in per-level tables (a horizontally uniform base state)
 # the mass fluxes read neither rho_b nor rho_b^w per cell, Kessler neither
 # theta_b, pi_b nor rho_b, the u, v step not theta_b.

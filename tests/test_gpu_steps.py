@@ -221,7 +221,7 @@ def test_acoustic_variants_are_bit_identical(name, prec, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec", ["f64", "f32"])
-@pytest.mark.parametrize("nx,ny,nz", [(16, 25, 44), (33, 20, 45), (17, 9, 31), (40, 12, 64)])
+@pytest.mark.parametrize("nx,ny,nz", [(16, 25, 44), (33, 20, 45), (17, 9, 31), (40, 12, 64), (9, 8, 5), (24, 6, 96)])
 def test_column_variants_over_a_hill_in_both_directions(nx, ny, nz, prec, monkeypatch):
     """Terrain sloping in x and in y under columns deeper and shallower than 32
     levels, ragged tiles: every acoustic variant gives the surface w = u h_x +

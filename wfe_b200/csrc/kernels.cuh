@@ -340,16 +340,10 @@ enum {
   TC_W, TC_PI, TC_TH, TC_TW, TC_TTH, TC_TPI, TC_AW, TC_KT3, TC_THBW, TC_DTHB,
   TC_QV, TC_QC, TC_QR, TC_QVB, TC_N
 };
-// Persistent, pipelined column kernel (dyn_acou_pipe.cu): one producer warp
-// streams each tile's input boxes (the TC_* fields above, levels 0..nz-1 and
-// w 0..nz) into a ring of shared-memory stages by bulk tensor loads while the
-// consumer warps run the column phases of the tile before; the same
-// expressions as the chunked kernel, bit for bit.  Maps are encoded with the
-// boxes of acoustic_pipe_box for the chosen shape.
 // The column inputs that depend on the level alone when the base state and
 // the metric are horizontally uniform (flat ground, one map factor): the
-// pipelined column kernels then read them from per-level tables, in this
-// order, instead of streaming a box of each per tile.
+// register-held and the pipelined column kernels then read them from
+// per-level tables, in this order, instead of the fields.
 enum { PF_RTJX = 0, PF_RTJY, PF_AW, PF_KT3, PF_THBW, PF_DTHB, PF_QVB, PF_N };
 WFE_HD int pipe_prof_slot(int f) {
   switch (f) {
@@ -371,23 +365,16 @@ struct PipeColParams {
   const R* prof;   // PF_N tables of nz + 1 levels, or null (boxes for all)
   CUtensorMap map[TC_N];
 };
-int acoustic_pipe_shapes();
-// box extents of field f (TC_*) for pipe shape `shape` and nz levels
-void acoustic_pipe_box(int shape, int f, int nz, int* bx, int* by, int* bz);
-// 0 when the shape's stages do not fit in shared memory
-template <typename R>
-size_t acoustic_pipe_smem(int shape, int nz, bool moist, bool tpi, bool prof = false);
+// Persistent, pipelined column kernel (dyn_acou_pipe.cu): one producer warp
+// streams each tile's input boxes (the TC_* fields above, levels 0..nz-1 and
+// w 0..nz) into a ring of shared-memory stages by bulk tensor loads while the
+// consumer warps solve the tile before with the parallel solve (level lanes
+// own consecutive rows in registers, cyclic reduction across the lanes: equal
+// to the Thomas kernels to rounding).  Maps are encoded with the boxes of
+// acoustic_pipe_pcr_box for the chosen shape.
 // raises every shape's shared-memory limit to the largest layout it may use
 template <typename R>
 int prepare_acoustic_pipe(int nz);
-// Returns 0 ok, 2 does not fit
-template <typename R>
-int launch_acoustic_column_pipe(const PipeColParams<R>& p, int shape, cudaStream_t st);
-// The same pipeline feeding the parallel-solve column (level lanes own
-// consecutive rows in registers, cyclic reduction across the lanes: equal to
-// the Thomas kernels to rounding); its own shapes, boxes and layouts, the
-// same params (maps encoded with acoustic_pipe_pcr_box).  prepare_acoustic_pipe
-// raises these kernels' limits too.
 int acoustic_pipe_pcr_shapes();
 void acoustic_pipe_pcr_box(int shape, int f, int nz, int* bx, int* by, int* bz);
 template <typename R>
@@ -445,13 +432,16 @@ template <typename R>
 bool acoustic_fused_fits(int nz, int f);
 template <typename R>
 int prepare_acoustic_fused(int nz);
-// The column kernel with contiguous level chunks per lane (fewer barriers),
-// acoustic_chunked_shapes() shapes; same values as launch_acoustic_column.
+// The column kernel with every level's inputs in registers (dyn_acou_reg.cu),
+// acoustic_reg_shapes() shapes; same values as launch_acoustic_column.  prof:
+// the per-level coefficient tables (PipeColParams::prof) or null.
 template <typename R>
-int launch_acoustic_column_chunked(const AcouArgs<R>& a, int f, cudaStream_t st);
-int acoustic_chunked_shapes();
+int launch_acoustic_column_reg(const AcouArgs<R>& a, const R* prof, int s, cudaStream_t st);
+int acoustic_reg_shapes();
 template <typename R>
-bool acoustic_chunked_fits(int nz, int f);
+bool acoustic_reg_fits(int nz, int s);
+template <typename R>
+int prepare_acoustic_reg(int nz);
 // The column kernel with a parallel (partitioned + cyclic-reduction)
 // tridiagonal solve, acoustic_pcr_shapes() shapes; the same rows as the
 // other column kernels, the solution equal to theirs up to rounding.

@@ -133,6 +133,7 @@ class ModelT final : public Model {
     if (prepare_acoustic_column<R>(g_.nz) || prepare_kessler<R>(g_.nz) || prepare_sfc<R>(g_.nz))
       return fail("nz too large for the column kernels' shared memory");
     fused_ok_ = prepare_acoustic_fused<R>(g_.nz) == 0;
+    reg_ok_ = prepare_acoustic_reg<R>(g_.nz) == 0;
     pipe_ok_ = tensor_map_encoder() && prepare_acoustic_pipe<R>(g_.nz) == 0;
     uvp_ok_ = tensor_map_encoder() && prepare_acoustic_uv_pipe<R>() == 0;
     tend_tma_ok_ = tensor_map_encoder() && tend_scal_tma_smem<R>() <= 227 * 1024 &&
@@ -774,45 +775,34 @@ class ModelT final : public Model {
     out[2] = tune_.done ? tune_.uv_variant : -1;
     out[3] = (lvl_tab_ != nullptr ? 1 : 0) | (db_.lvl != nullptr ? 2 : 0);
   }
-  // chunked column variants follow the fused ones; -1 for other variants
-  int chunked_index(int v) const {
+  // column variants by number: the tile shapes, one number that is free, the
+  // fused substep kernels, the register-held columns, the parallel solve and
+  // its pipelined form; an index is -1 for a variant of another kind
+  int reg_index(int v) const {
     const int f = v - acoustic_column_shapes() - 1 - acoustic_fused_shapes();
-    return (f >= 0 && f < acoustic_chunked_shapes()) ? f : -1;
+    return (f >= 0 && f < acoustic_reg_shapes()) ? f : -1;
   }
-  bool chunked_usable(int v) const {
-    const int f = chunked_index(v);
-    return f >= 0 && acoustic_chunked_fits<R>(g_.nz, f);
+  bool reg_usable(int v) const {
+    const int f = reg_index(v);
+    return f >= 0 && reg_ok_ && acoustic_reg_fits<R>(g_.nz, f);
   }
-  // pipelined column variants follow the chunked ones; -1 for other variants
-  int pipe_index(int v) const {
-    const int f = v - acoustic_column_shapes() - 1 - acoustic_fused_shapes() - acoustic_chunked_shapes();
-    return (f >= 0 && f < acoustic_pipe_shapes()) ? f : -1;
-  }
-  // parallel-solve column variants follow the pipelined ones; -1 otherwise
   int pcr_index(int v) const {
-    const int f = v - acoustic_column_shapes() - 1 - acoustic_fused_shapes() - acoustic_chunked_shapes() -
-                  acoustic_pipe_shapes();
+    const int f = v - acoustic_column_shapes() - 1 - acoustic_fused_shapes() - acoustic_reg_shapes();
     return (f >= 0 && f < acoustic_pcr_shapes()) ? f : -1;
   }
   bool pcr_usable(int v) const {
     const int f = pcr_index(v);
     return f >= 0 && acoustic_pcr_fits<R>(g_.nz, f);
   }
-  // pipelined parallel-solve column variants follow those; -1 otherwise
   int pipe_pcr_index(int v) const {
-    const int f = v - acoustic_column_shapes() - 1 - acoustic_fused_shapes() - acoustic_chunked_shapes() -
-                  acoustic_pipe_shapes() - acoustic_pcr_shapes();
+    const int f = v - acoustic_column_shapes() - 1 - acoustic_fused_shapes() - acoustic_reg_shapes() -
+                  acoustic_pcr_shapes();
     return (f >= 0 && f < acoustic_pipe_pcr_shapes()) ? f : -1;
   }
   bool pipe_pcr_usable(int v) const {
     const int f = pipe_pcr_index(v);
     return pipe_ok_ && f >= 0 &&
            acoustic_pipe_pcr_smem<R>(f, g_.nz, dp_.moisture != 0, bdy_on_, lvl_tab_ != nullptr) > 0;
-  }
-  bool pipe_usable(int v) const {
-    const int f = pipe_index(v);
-    return pipe_ok_ && f >= 0 &&
-           acoustic_pipe_smem<R>(f, g_.nz, dp_.moisture != 0, bdy_on_, lvl_tab_ != nullptr) > 0;
   }
   bool fused_usable(int v) const {
     const int f = v - acoustic_column_shapes() - 1;
@@ -855,7 +845,7 @@ class ModelT final : public Model {
     std::string name = prop.name;
     for (char& ch : name)
       if (ch == ' ') ch = '_';
-    k << "v9|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
+    k << "v10|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
       << dp_.moisture << "pd" << dp_.pd_moist << "b" << bdy_on_ << "d" << (dp_.diff_K > 0) << "x"
       << (pcr_allowed() ? 0 : 1);
     return k.str();
@@ -900,8 +890,8 @@ class ModelT final : public Model {
 
   // WFE_COLUMN_VARIANT=<n> forces the acoustic variant (0..5 column tile
   // shapes, 6 the first of them again -- the number of a kernel that is
-  // gone --, 7..9 the fused substep kernel in three tile shapes, 10..12 the chunked column kernel, 13..15 the persistent
-  // pipelined column kernel, 16..18 the parallel-solve column kernel and
+  // gone --, 7..9 the fused substep kernel in three tile shapes, 10..15 the register-held
+  // column kernel in six shapes, 16..18 the parallel-solve column kernel and
   // 19..22 its pipelined form, both equal to the others up to rounding),
   // WFE_UV_VARIANT=<n> the forward u, v kernel (0
   // thread per face pair in 16 x 16 x 1 blocks, 1 persistent pipelined tiles,
@@ -915,8 +905,8 @@ class ModelT final : public Model {
     const char* cv = std::getenv("WFE_COLUMN_VARIANT");
     if (first && cv && *cv) {
       const int v = std::atoi(cv);
-      if (v >= 0 && (v <= acoustic_column_shapes() || fused_usable(v) || chunked_usable(v) || pipe_usable(v) ||
-                     pcr_usable(v) || pipe_pcr_usable(v)))
+      if (v >= 0 && (v <= acoustic_column_shapes() || fused_usable(v) || reg_usable(v) || pcr_usable(v) ||
+                     pipe_pcr_usable(v)))
         tune_.column_cx = v;
     }
     const char* uvv = std::getenv("WFE_UV_VARIANT");
@@ -978,11 +968,11 @@ class ModelT final : public Model {
     tune_.uv_variant = cached.uv_variant;
     best = 1e30f;
     // tile shapes, the fused substep kernels (number 6 stays free)
-    const int nvar = acoustic_column_shapes() + 1 + acoustic_fused_shapes() + acoustic_chunked_shapes() +
-                     acoustic_pipe_shapes() + acoustic_pcr_shapes() + acoustic_pipe_pcr_shapes();
+    const int nvar = acoustic_column_shapes() + 1 + acoustic_fused_shapes() + acoustic_reg_shapes() +
+                     acoustic_pcr_shapes() + acoustic_pipe_pcr_shapes();
     for (int cx = 0; cx < nvar; ++cx) {
-      if (cx >= acoustic_column_shapes() && !fused_usable(cx) && !chunked_usable(cx) &&
-          !pipe_usable(cx) && !pcr_usable(cx) && !pipe_pcr_usable(cx))
+      if (cx >= acoustic_column_shapes() && !fused_usable(cx) && !reg_usable(cx) && !pcr_usable(cx) &&
+          !pipe_pcr_usable(cx))
         continue;
       // the parallel-solve variants agree with the others to rounding only:
       // the tuner picks them only where allowed (WFE_EXACT_COLUMN=0)
@@ -1155,9 +1145,9 @@ class ModelT final : public Model {
   int column_launch(const AcouArgs<R>& a, int v) {
     if (fused_usable(v)) v = acoustic_fused_column_shape(v - acoustic_column_shapes() - 1);
     int rc = 0;
-    if (chunked_usable(v)) {
-      const int f = chunked_index(v);
-      launch("acoustic_column", [&] { rc = launch_acoustic_column_chunked<R>(a, f, st_); });
+    if (reg_usable(v)) {
+      const int f = reg_index(v);
+      launch("acoustic_column", [&] { rc = launch_acoustic_column_reg<R>(a, lvl_tab_, f, st_); });
     } else if (pcr_usable(v)) {
       const int f = pcr_index(v);
       launch("acoustic_column", [&] { rc = launch_acoustic_column_pcr<R>(a, f, st_); });
@@ -1166,17 +1156,8 @@ class ModelT final : public Model {
                                          lvl_tab_ != nullptr) > 0) {
       const int f = pipe_pcr_index(v);
       PipeColParams<R> pp;
-      if (pipe_params(a, f, &pp, true)) return 1;
-      launch("acoustic_column", [&] { rc = launch_acoustic_column_pipe_pcr<R>(pp, f, st_); });
-    } else if (pipe_usable(v) &&
-               acoustic_pipe_smem<R>(pipe_index(v), g_.nz, dp_.moisture != 0, a.tpi != nullptr,
-                                     lvl_tab_ != nullptr) > 0) {
-      // (operator-level calls add the slow pi' tendency box: when that no
-      // longer fits, the plain column kernel below takes the launch)
-      const int f = pipe_index(v);
-      PipeColParams<R> pp;
       if (pipe_params(a, f, &pp)) return 1;
-      launch("acoustic_column", [&] { rc = launch_acoustic_column_pipe<R>(pp, f, st_); });
+      launch("acoustic_column", [&] { rc = launch_acoustic_column_pipe_pcr<R>(pp, f, st_); });
     } else {
       launch("acoustic_column",
              [&] { rc = launch_acoustic_column<R>(a, v < acoustic_column_shapes() ? v : 0, st_); });
@@ -1317,8 +1298,7 @@ class ModelT final : public Model {
     return 0;
   }
 
-  // pcr: the boxes of the pipelined parallel-solve shapes
-  int pipe_params(const AcouArgs<R>& a, int shape, PipeColParams<R>* pp, bool pcr = false) {
+  int pipe_params(const AcouArgs<R>& a, int shape, PipeColParams<R>* pp) {
     std::memset(static_cast<void*>(pp), 0, sizeof(*pp));
     pp->a = a;
     pp->err = tma_err_;
@@ -1332,10 +1312,7 @@ class ModelT final : public Model {
       if (f >= TC_QV && !a.p.moisture) continue;
       if (pp->prof && pipe_prof_slot(f) >= 0) continue;
       int bx, by, bz;
-      if (pcr)
-        acoustic_pipe_pcr_box(shape, f, g_.nz, &bx, &by, &bz);
-      else
-        acoustic_pipe_box(shape, f, g_.nz, &bx, &by, &bz);
+      acoustic_pipe_pcr_box(shape, f, g_.nz, &bx, &by, &bz);
       const CUtensorMap* m = tmap3(src[f], bx, by, bz);
       if (!m) return 1;
       pp->map[f] = *m;
@@ -1643,6 +1620,7 @@ class ModelT final : public Model {
   long gen_ = 0;  // changes whenever buffer roles or physics switches change
   std::vector<Rec>* rec_ = nullptr;  // record mode when set
   bool fused_ok_ = false;            // fused substep kernels prepared
+  bool reg_ok_ = false;              // register-held column variants usable
   bool pipe_ok_ = false;             // pipelined column kernels prepared
   bool uvp_ok_ = false;              // pipelined u, v kernel prepared
   bool tend_tma_ok_ = false;         // TMA-staged scalar tendencies usable
