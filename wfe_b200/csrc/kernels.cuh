@@ -271,7 +271,7 @@ int lin_kessler_prepare(int nz);
 // copy `count` whole fields of n elements each (src[f] -> dst[f]) in one
 // launch; 16-byte aligned pointers and n * sizeof(R) a multiple of 16, else
 // nothing is launched and 1 is returned
-constexpr int kCopyMax = 8;
+constexpr int kCopyMax = 20;
 template <typename R>
 struct CopyJob {
   const R* src[kCopyMax];

@@ -889,73 +889,123 @@ __global__ void __launch_bounds__(256, kUvLinMinBlocks<R>) k_ad_uv_cells(AcouArg
 }
 
 // ================================================================ w - pi' column
-// A CTA owns kLcx columns of one row with kLkl level lanes; the column arrays
+// A CTA owns kLcx columns of one row with blockDim.y level lanes; the column arrays
 // live in shared memory ([level * kLcx + column]); the sweeps run in one lane
 // per column, everything else in parallel over the levels.
-// FP32 tiles hold 16 columns x 8 level lanes; FP64 keeps 8 columns x 16 lanes
-// so that the adjoint's arrays for lin_max_levels() levels fit in shared memory
+// FP32 tiles hold 16 columns, FP64 8, so that the adjoint's arrays for
+// lin_max_levels() levels fit in shared memory; the level lanes beside them
+// are chosen per launch (lin_lanes)
 template <typename R>
 constexpr int kLcx = sizeof(R) == 4 ? 16 : 8;
-template <typename R>
-constexpr int kLkl = sizeof(R) == 4 ? 8 : 16;
+constexpr int kLinColThreads = 512;
 
-// rows 1..n-1 of a tridiagonal system (row 1 without A, row n-1 without C),
-// the forward's elimination (kernels.cu:612-634; dyn_acou.cu phase 4: one
-// reciprocal per row); arrays strided by kLcx<R>
+// Tridiagonal sweeps over rows 1..n-1 (row 1 without the lower, row n-1
+// without the upper coefficient) in one thread, arrays strided by kLcx<R>:
+// the forward's elimination (kernels.cu:612-634; one reciprocal per row).
+// One warp sweeps while the CTA waits, so its latency is the launch's: rows
+// are read four at a time ahead of the chain that uses them, and the way
+// back eight.
 template <typename R>
-__device__ __forceinline__ void thomas_s(int n, const R* A, const R* B, const R* C, const R* D, R* cs, R* ds,
-                                         R* x) {
-  R cp = 0, dp = 0;
-  for (int k = 1; k < n; ++k) {
-    const int q = k * kLcx<R>;
-    if (k == 1) {
-      const R r = (R)1 / B[q];
-      cp = C[q] * r;
-      dp = D[q] * r;
-    } else {
-      const R r = (R)1 / (B[q] - A[q] * cp);
-      cp = C[q] * r;
-      dp = (D[q] - A[q] * dp) * r;
-    }
-    cs[q] = cp;
-    ds[q] = dp;
-  }
-  x[n * kLcx<R>] = 0;
+__device__ __forceinline__ void back_substitute(int n, const R* cs, const R* ds, R* x) {
+  constexpr int X = kLcx<R>;
+  x[n * X] = 0;
   R above = 0;
-  for (int k = n - 1; k >= 1; --k) {
-    above = ds[k * kLcx<R>] - cs[k * kLcx<R>] * above;
-    x[k * kLcx<R>] = above;
+  int k = n - 1;
+  for (; k >= 8; k -= 8) {
+    R c[8], d[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = cs[(k - q) * X], d[q] = ds[(k - q) * X];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      above = d[q] - c[q] * above;
+      x[(k - q) * X] = above;
+    }
   }
+  for (; k >= 1; --k) {
+    above = ds[k * X] - cs[k * X] * above;
+    x[k * X] = above;
+  }
+}
+
+// low(k), up(k): the row's lower and upper coefficient.  RINV keeps the rows'
+// reciprocals for resolve_s.
+template <typename R, class Low, class Up, bool RINV>
+__device__ __forceinline__ void eliminate(int n, Low low, const R* B, Up up, const R* D, R* cs, R* ds, R* rinv) {
+  constexpr int X = kLcx<R>;
+  R a[4], b[4], c[4], d[4];
+  auto rows = [&](int kb) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = kb + q < n ? kb + q : n - 1;
+      a[q] = low(k), b[q] = B[k * X], c[q] = up(k), d[q] = D[k * X];
+    }
+  };
+  rows(1);
+  a[0] = 0;
+  R cp = 0, dp = 0;
+  for (int kb = 1; kb < n; kb += 4) {
+    R a0[4], b0[4], c0[4], d0[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a0[q] = a[q], b0[q] = b[q], c0[q] = c[q], d0[q] = d[q];
+    rows(kb + 4);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const R r = (R)1 / (b0[q] - a0[q] * cp);
+      cp = c0[q] * r;
+      dp = (d0[q] - a0[q] * dp) * r;
+      if (kb + q < n) {
+        cs[(kb + q) * X] = cp;
+        ds[(kb + q) * X] = dp;
+        if (RINV) rinv[(kb + q) * X] = r;
+      }
+    }
+  }
+}
+
+// rinv: null, or where the rows' reciprocals go (not one of the inputs)
+template <typename R, bool RINV = false>
+__device__ __forceinline__ void thomas_s(int n, const R* A, const R* B, const R* C, const R* D, R* cs, R* ds,
+                                         R* x, R* rinv = nullptr) {
+  constexpr int X = kLcx<R>;
+  auto low = [&](int k) { return A[k * X]; };
+  auto up = [&](int k) { return C[k * X]; };
+  eliminate<R, decltype(low), decltype(up), RINV>(n, low, B, up, D, cs, ds, rinv);
+  back_substitute(n, cs, ds, x);
+}
+
+// the same matrix once more: its eliminated rows cs and reciprocals from
+// thomas_s, another right-hand side (the values thomas_s would give, without
+// its chain of reciprocals)
+template <typename R>
+__device__ __forceinline__ void resolve_s(int n, const R* A, const R* rinv, const R* D, const R* cs, R* ds, R* x) {
+  constexpr int X = kLcx<R>;
+  R dp = 0;
+  for (int kb = 1; kb < n; kb += 8) {
+    R a[8], r[8], d[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int k = kb + q < n ? kb + q : n - 1;
+      a[q] = k > 1 ? A[k * X] : (R)0, r[q] = rinv[k * X], d[q] = D[k * X];
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      dp = (d[q] - a[q] * dp) * r[q];
+      if (kb + q < n) ds[(kb + q) * X] = dp;
+    }
+  }
+  back_substitute(n, cs, ds, x);
 }
 
 // the transposed system: (M^T)_{k,k-1} = C[k-1], (M^T)_{k,k+1} = A[k+1]
 template <typename R>
 __device__ __forceinline__ void thomas_ts(int n, const R* A, const R* B, const R* C, const R* D, R* cs, R* ds,
                                           R* x) {
-  R cp = 0, dp = 0;
-  for (int k = 1; k < n; ++k) {
-    const int q = k * kLcx<R>;
-    const R sub = k > 1 ? C[q - kLcx<R>] : (R)0;
-    const R sup = k < n - 1 ? A[q + kLcx<R>] : (R)0;
-    if (k == 1) {
-      const R r = (R)1 / B[q];
-      cp = sup * r;
-      dp = D[q] * r;
-    } else {
-      const R r = (R)1 / (B[q] - sub * cp);
-      cp = sup * r;
-      dp = (D[q] - sub * dp) * r;
-    }
-    cs[q] = cp;
-    ds[q] = dp;
-  }
-  x[n * kLcx<R>] = 0;
+  constexpr int X = kLcx<R>;
+  auto low = [&](int k) { return C[(k - 1) * X]; };
+  auto up = [&](int k) { return k < n - 1 ? A[(k + 1) * X] : (R)0; };
+  eliminate<R, decltype(low), decltype(up), false>(n, low, B, up, D, cs, ds, nullptr);
   x[0] = 0;
-  R above = 0;
-  for (int k = n - 1; k >= 1; --k) {
-    above = ds[k * kLcx<R>] - cs[k * kLcx<R>] * above;
-    x[k * kLcx<R>] = above;
-  }
+  back_substitute(n, cs, ds, x);
 }
 
 // shared column arrays: a fixed set of (nz + 1)-level arrays
@@ -1003,9 +1053,10 @@ struct ColGeom {
 // surface w at level 0).  Ends with a barrier.
 enum { V_AV, V_SV, V_P, V_E, V_G, V_A, V_B, V_C, V_D, V_W, V_CS, V_DS, V_N };
 
-template <typename R>
+// RINV: the rows' reciprocals into array `rinv` for a second solve.
+template <typename R, bool RINV = false>
 __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColGeom<R>& g, bool active,
-                                                const ColArr<R>& S) {
+                                                const ColArr<R>& S, int rinv = 0) {
   const Layout& L = a.L;
   const int nz = g.nz, tx = threadIdx.x, lane = threadIdx.y;
   const R dtau = g.dtau, c1 = g.c1, c2 = g.c2;
@@ -1016,7 +1067,7 @@ __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColG
   R *G = S[V_G] + tx, *A = S[V_A] + tx, *B = S[V_B] + tx, *C = S[V_C] + tx, *D = S[V_D] + tx;
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       R av = 0, sv = 0;
       if (k >= 1 && k < nz) {
         const int c = g.at(k), cm = c - pl;
@@ -1033,7 +1084,7 @@ __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColG
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = lane; k < nz; k += kLkl<R>) {
+    for (int k = lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       R Kt = a.co.kt3[c];
       R Dh = (a.co.rtjx[c + sx] * u[c + sx] - a.co.rtjx[c] * u[c]) * g.mcx +
@@ -1049,7 +1100,7 @@ __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColG
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = 1 + lane; k < nz; k += kLkl<R>) {
+    for (int k = 1 + lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k), cm = c - pl;
       const R iJdz = g.invJ * a.co.inv_dzw[L.at1(k)];
       R thc = a.th_in[c], thm = a.th_in[cm];
@@ -1076,7 +1127,7 @@ __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColG
   __syncthreads();
   if (active && lane == 0) {
     R* W = S[V_W] + tx;
-    thomas_s(nz, A, B, C, D, S[V_CS] + tx, S[V_DS] + tx, W);
+    thomas_s<R, RINV>(nz, A, B, C, D, S[V_CS] + tx, S[V_DS] + tx, W, RINV ? S[rinv] + tx : nullptr);
     R us = (R)0.5 * (u[g.c0] + u[g.c0 + sx]);
     R vs = (R)0.5 * (v[g.c0] + v[g.c0 + sy]);
     W[0] = us * g.hxc + vs * g.hyc;
@@ -1101,7 +1152,7 @@ __device__ __forceinline__ void column_values_stored_s(const AcouArgs<R>& a, con
   R *G = S[V_G] + tx, *A = S[V_A] + tx, *B = S[V_B] + tx, *C = S[V_C] + tx;
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       Av[k * kLcx<R>] = (k >= 1 && k < nz) ? a.co.aw[c] : (R)0;
       W[k * kLcx<R>] = k < nz ? a.w_out[c] : (R)0;
@@ -1109,7 +1160,7 @@ __device__ __forceinline__ void column_values_stored_s(const AcouArgs<R>& a, con
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = lane; k < nz; k += kLkl<R>) {
+    for (int k = lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       const int q = k * kLcx<R>;
       const R e = dtau * a.co.kt3[c] * c1 * a.co.inv_dzc[L.at1(k)];
@@ -1119,7 +1170,7 @@ __device__ __forceinline__ void column_values_stored_s(const AcouArgs<R>& a, con
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = 1 + lane; k < nz; k += kLkl<R>) {
+    for (int k = 1 + lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k), cm = c - g.pl;
       const R iJdz = g.invJ * a.co.inv_dzw[L.at1(k)];
       R thvw = a.b.thbw[c] + (R)0.5 * (a.th_in[cm] + a.th_in[c]);
@@ -1135,10 +1186,10 @@ __device__ __forceinline__ void column_values_stored_s(const AcouArgs<R>& a, con
   __syncthreads();
 }
 
-enum { T_DSV = V_N, T_DTH, T_DP, T_RHS, T_DW, T_NARR };
+enum { T_DSV = V_N, T_DTH, T_DP, T_RHS, T_DW, T_RINV, T_NARR };
 
 template <typename R>
-__global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_tl_column(AcouArgs<R> a, AcouArgs<R> d, int with_forward) {
+__global__ void __launch_bounds__(kLinColThreads) k_tl_column(AcouArgs<R> a, AcouArgs<R> d, int with_forward) {
   extern __shared__ __align__(16) unsigned char lin_smem[];
   const Layout& L = a.L;
   const int tx = threadIdx.x, lane = threadIdx.y;
@@ -1156,13 +1207,13 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_tl_column(AcouArgs<R> a, 
   // the tangent theta' in, before any in-place write of this launch
   if (active)
 #pragma unroll 4
-    for (int k = lane; k < nz; k += kLkl<R>) dth[k * kLcx<R>] = d.th_in[g.at(k)];
-  column_values_s(a, g, active, S);
+    for (int k = lane; k < nz; k += (int)blockDim.y) dth[k * kLcx<R>] = d.th_in[g.at(k)];
+  column_values_s<R, true>(a, g, active, S, T_RINV);
   const R *Av = S[V_AV] + tx, *P = S[V_P] + tx, *E = S[V_E] + tx, *G = S[V_G] + tx;
   const R* W = S[V_W] + tx;
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       R sv = 0;
       if (g.terrain && k >= 1 && k < nz) {
         const int c = g.at(k), cm = c - pl;
@@ -1175,7 +1226,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_tl_column(AcouArgs<R> a, 
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = lane; k < nz; k += kLkl<R>) {
+    for (int k = lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       R Kt = a.co.kt3[c];
       R dDh = (a.co.rtjx[c + sx] * du[c + sx] - a.co.rtjx[c] * du[c]) * g.mcx +
@@ -1190,7 +1241,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_tl_column(AcouArgs<R> a, 
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = 1 + lane; k < nz; k += kLkl<R>) {
+    for (int k = 1 + lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k), cm = c - pl;
       const int q = k * kLcx<R>;
       const R iJdz = g.invJ * a.co.inv_dzw[L.at1(k)];
@@ -1221,13 +1272,13 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_tl_column(AcouArgs<R> a, 
     }
   __syncthreads();
   if (active && lane == 0) {
-    thomas_s(nz, S[V_A] + tx, S[V_B] + tx, S[V_C] + tx, rhs, S[V_CS] + tx, S[V_DS] + tx, dw);
+    resolve_s(nz, S[V_A] + tx, S[T_RINV] + tx, rhs, S[V_CS] + tx, S[V_DS] + tx, dw);
     dw[0] = (R)0.5 * (du[g.c0] + du[g.c0 + sx]) * g.hxc + (R)0.5 * (dv[g.c0] + dv[g.c0 + sy]) * g.hyc;
   }
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       const int q = k * kLcx<R>;
       if (k < nz) {
@@ -1262,7 +1313,7 @@ enum { A_WB = V_N, A_PB, A_TB, A_WS, A_LAM, A_GL, A_PIB, A_THB, A_KTD, A_NARR };
 // STORED: the forward values from the launch's outputs (column_values_stored_s)
 // instead of recomputing the forward column
 template <typename R, bool STORED = false>
-__global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_ad_column(AcouArgs<R> a, AcouArgs<R> d, R* dhB, R* svB) {
+__global__ void __launch_bounds__(kLinColThreads) k_ad_column(AcouArgs<R> a, AcouArgs<R> d, R* dhB, R* svB) {
   extern __shared__ __align__(16) unsigned char lin_smem[];
   const Layout& L = a.L;
   const int tx = threadIdx.x, lane = threadIdx.y;
@@ -1297,7 +1348,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_ad_column(AcouArgs<R> a, 
   const bool w_alias = d.w_out == d.w_in, th_alias = d.th_out == d.th_in;
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       const int q = k * kLcx<R>;
       wb[q] = d.w_out[c];
@@ -1315,7 +1366,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_ad_column(AcouArgs<R> a, 
   // adjoint of the column solution w (level 0: surface w, level nz: the lid)
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       const int q = k * kLcx<R>;
       const int c = g.at(k);
       R s = 0;
@@ -1330,7 +1381,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_ad_column(AcouArgs<R> a, 
   // per inner level: what its row sends to neighbouring levels
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       const int q = k * kLcx<R>;
       if (k < 1 || k >= nz) {
         GL[q] = 0;
@@ -1365,7 +1416,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_ad_column(AcouArgs<R> a, 
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = lane; k < nz; k += kLkl<R>) {
+    for (int k = lane; k < nz; k += (int)blockDim.y) {
       const int c = g.at(k);
       const int q = k * kLcx<R>;
       // the adjoints this level accumulates into, all read first
@@ -1409,7 +1460,7 @@ __global__ void __launch_bounds__(kLcx<R> * kLkl<R>) k_ad_column(AcouArgs<R> a, 
   __syncthreads();
   if (active)
 #pragma unroll 4
-    for (int k = lane; k <= nz; k += kLkl<R>) {
+    for (int k = lane; k <= nz; k += (int)blockDim.y) {
       const int q = k * kLcx<R>;
       const int c = g.at(k);
       const R w0 = w_alias ? (R)0 : wI[c];
@@ -1560,6 +1611,17 @@ void ad_uv(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr,
   k_ad_uv_cells<R><<<grid_cells<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, w);
 }
 
+// Level lanes of a column CTA: 16, or 32 where the grid gives an SM at most
+// two CTAs (nothing else is resident to hide a lane's serial levels).
+// Tangent-linear run per step, FP32, 8 / 16 / 32 lanes: 400x4x65 slab (100
+// CTAs) 0.71 / 0.60 / 0.56 ms, 96x96x40 1.20 / 1.16 / 1.30, 160x160x40 3.1 /
+// 2.9 / 3.4; adjoint run of the slab 1.21 / 1.12 / 1.10.
+template <typename R>
+static int lin_lanes(const Layout& L) {
+  constexpr int kFewCtas = 2 * 148;
+  return (L.nx + kLcx<R> - 1) / kLcx<R> * L.ny <= kFewCtas ? 32 : 16;
+}
+
 int lin_max_levels() { return 160; }  // FP64 adjoint column arrays within 227 KB
 
 template <typename R, int NARR>
@@ -1583,7 +1645,7 @@ template <typename R>
 int tl_column(const AcouArgs<R>& a, const AcouArgs<R>& d, bool with_forward, cudaStream_t st) {
   if (a.L.nz > lin_max_levels()) return 2;
   const size_t sm = lin_col_smem<R, T_NARR>(a.L.nz);
-  k_tl_column<R><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, kLkl<R>), sm, st>>>(
+  k_tl_column<R><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, lin_lanes<R>(a.L)), sm, st>>>(
       a, d, with_forward ? 1 : 0);
   return 0;
 }
@@ -1592,7 +1654,7 @@ template <typename R>
 int ad_column(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
   if (a.L.nz > lin_max_levels()) return 2;
   const size_t sm = lin_col_smem<R, A_NARR>(a.L.nz);
-  k_ad_column<R><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, kLkl<R>), sm, st>>>(a, d, scr.f[0], scr.f[1]);
+  k_ad_column<R><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, lin_lanes<R>(a.L)), sm, st>>>(a, d, scr.f[0], scr.f[1]);
   k_ad_column_uv<R><<<grid_uv<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, scr.f[0], scr.f[1]);
   return 0;
 }
@@ -1601,7 +1663,7 @@ template <typename R>
 int ad_column_stored(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
   if (a.L.nz > lin_max_levels()) return 2;
   const size_t sm = lin_col_smem<R, A_NARR>(a.L.nz);
-  k_ad_column<R, true><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, kLkl<R>), sm, st>>>(
+  k_ad_column<R, true><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, lin_lanes<R>(a.L)), sm, st>>>(
       a, d, scr.f[0], scr.f[1]);
   k_ad_column_uv<R><<<grid_uv<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, scr.f[0], scr.f[1]);
   return 0;

@@ -520,44 +520,74 @@ class LinT final : public Lin {
     if (!rain_scratch_) LCK(cudaMalloc(&rain_scratch_, L_.n2() * sizeof(R)));
     if (slots > log_cap_) return fail("undo log smaller than the segment (ensure_log not called)");
     SegGraphs g;
+    // The launches in groups that share one undo-log copy each way: a stage's
+    // fill, mass fluxes and tendencies; a substep's u, v and column; Kessler.
+    // Within a group no launch reads what an earlier one of it overwrites but
+    // the step itself (fill -> fluxes -> tendencies, u, v -> column), so every
+    // output can be saved before the group's first launch, and the group's
+    // adjoints -- which read the values the forward launches left -- run
+    // before its outputs are restored.  The u, v adjoint alone reads fields
+    // its substep's column replaced (w, pi', theta'): the group's restore goes
+    // between the two.
+    struct Group {
+      size_t step, first, last;  // launches [first, last] of a step
+      std::vector<R*> out;       // what they overwrite, launch by launch
+      size_t slot;               // their place in the log
+      size_t at_last;            // slots of the group before the last launch's
+    };
+    std::vector<Group> groups;
+    size_t slot0 = 0;
+    for (size_t s = 0; s < recs.size(); ++s)
+      for (size_t q = 0; q < recs[s].size(); ++q) {
+        const int kind = recs[s][q].kind;
+        const bool follows = q > 0 && !groups.empty() && groups.back().step == s &&
+                             (kind == K_FLUX || kind == K_TEND || kind == K_COL);
+        if (!follows) groups.push_back(Group{s, q, q, {}, slot0, 0});
+        Group& gr = groups.back();
+        gr.last = q;
+        gr.at_last = gr.out.size();
+        outputs(recs[s][q], &o);
+        gr.out.insert(gr.out.end(), o.begin(), o.end());
+        slot0 += o.size();
+        if ((int)gr.out.size() > kCopyMax) return fail("undo-log group larger than a copy job");
+      }
+    auto copy = [&](const Group& gr, bool save) {
+      CopyJob<R> job{};
+      for (size_t z = 0; z < gr.out.size(); ++z) {
+        R* at = log_ + (gr.slot + z) * n3_;
+        job.src[job.count] = save ? gr.out[z] : at;
+        job.dst[job.count++] = save ? at : gr.out[z];
+      }
+      return copy_fields<R>(job, n3_, st_) ? fail("undo-log copy") : 0;
+    };
     if (capture(&g.fwd, [&] {
-          size_t slot = 0;
-          std::vector<R*> oo;
-          for (auto& st : recs)
-            for (const Rec& r : st) {
-              outputs(r, &oo);
-              CopyJob<R> job{};
-              for (R* p : oo) {
-                job.src[job.count] = p;
-                job.dst[job.count++] = log_ + slot * n3_;
-                ++slot;
-              }
-              if (copy_fields<R>(job, n3_, st_)) return fail("undo-log copy");
-              if (fwd(r, true)) return 1;
-            }
+          for (const Group& gr : groups) {
+            if (copy(gr, true)) return 1;
+            for (size_t q = gr.first; q <= gr.last; ++q)
+              if (fwd(recs[gr.step][q], true)) return 1;
+          }
           return 0;
         }))
       return 1;
     if (capture(&g.rev, [&] {
-          size_t slot = slots;
-          std::vector<R*> oo;
-          for (size_t s = recs.size(); s-- > 0;)
-            for (size_t q = recs[s].size(); q-- > 0;) {
-              const Rec& r = recs[s][q];
-              outputs(r, &oo);
-              // a column launch's adjoint runs before its outputs are
-              // restored: it reads the forward solution from them
-              const bool col = r.kind == K_COL;
-              if (col && ad_column_from_outputs(r, slot - oo.size())) return 1;
-              CopyJob<R> job{};
-              for (size_t z = oo.size(); z-- > 0;) {
-                --slot;
-                job.src[job.count] = log_ + slot * n3_;
-                job.dst[job.count++] = oo[z];
-              }
-              if (copy_fields<R>(job, n3_, st_)) return fail("undo-log copy");
-              if (!col && ad(r)) return 1;
+          for (size_t n = groups.size(); n-- > 0;) {
+            const Group& gr = groups[n];
+            const Rec& r = recs[gr.step][gr.last];
+            if (r.kind == K_COL) {
+              if (ad_column_from_outputs(r, gr.slot + gr.at_last) || copy(gr, false)) return 1;
+              for (size_t q = gr.last; q-- > gr.first;)
+                if (ad(recs[gr.step][q])) return 1;
+            } else if (r.kind == K_TEND) {
+              for (size_t q = gr.last + 1; q-- > gr.first;)
+                if (ad(recs[gr.step][q])) return 1;
+              if (copy(gr, false)) return 1;
+            } else {
+              // Kessler updates its inputs in place: restored first
+              if (copy(gr, false)) return 1;
+              for (size_t q = gr.last + 1; q-- > gr.first;)
+                if (ad(recs[gr.step][q])) return 1;
             }
+          }
           return 0;
         }))
       return 1;
