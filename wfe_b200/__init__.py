@@ -242,9 +242,9 @@ class Case:
         fid = FIELD_ID[name]
         if interior:
             nzl = self.nz + 1 if name == "w" else self.nz
-            out = np.zeros((nzl, self.ny, self.nx), dtype=dtype)
+            out = np.empty((nzl, self.ny, self.nx), dtype=dtype)
         else:
-            out = np.zeros(self.shape, dtype=dtype)
+            out = np.empty(self.shape, dtype=dtype)
         self._check(self._lib.wfe_field_download(
             self._h, ROLES[role], fid, out.ctypes.data_as(C.c_void_p),
             1 if dtype == np.float32 else 0, 1 if interior else 0))
