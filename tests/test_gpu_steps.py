@@ -268,6 +268,31 @@ def test_uv_variants_are_bit_identical(name, prec, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("bc", ["open", "periodic"])
+@pytest.mark.parametrize("nx,ny,nz", [(33, 9, 10), (34, 17, 11), (7, 8, 12), (64, 5, 9), (3, 4, 8), (40, 26, 4)])
+def test_uv_marches_over_a_hill(nx, ny, nz, bc, prec, monkeypatch):
+    """The column marches of the forward u, v step (1: two levels, 3: one) at the
+    edges of their 32 x 8 tiles and level pairs, with terrain sloping in x and y,
+    moisture, open and periodic boundaries, down to grids of the ghost width and
+    two interior levels: the same values, bit for bit, as the thread-per-face kernel (0)."""
+    ov = {"nx": str(nx), "ny": str(ny), "nz": str(nz), "dz": "500", "dt": "2", "stretch": "none", "bc_x": bc, "bc_y": bc}
+    out = {}
+    for v in ("0", "1", "2", "3"):
+        monkeypatch.setenv("WFE_UV_VARIANT", v)
+        c = W.Case(CASES / "ops_open.ini", ov, precision=prec)
+        for s in range(2):
+            c.step(c.dt, s * c.dt)
+        out[v] = {k: c.field(k) for k in W.FIELDS}
+        assert c.variants()["uv"] == int(v)
+        c.close()
+    assert np.isfinite(out["0"]["u"]).all()
+    for v in ("1", "2", "3"):
+        for k in W.FIELDS:
+            assert np.array_equal(out["0"][k], out[v][k]), (v, k)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name", ["wk82_small", "schaer_open", "straka_periodic", "bubble_open"])
 @pytest.mark.parametrize("prec", ["f64", "f32"])
 def test_tendency_variants_are_bit_identical(name, prec, monkeypatch):

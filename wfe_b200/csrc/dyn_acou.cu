@@ -457,182 +457,179 @@ __global__ void __launch_bounds__(256, kUvMinBlocks<R>) k_acoustic_uv_batch(Batc
   for_each_work(b, [](const AcouArgs<R>& a, int x, int y, int z) { uv_body(a, x, y, z); });
 }
 
-// ------------------------------------------ pipelined forward u, v
-// Persistent CTAs over tiles of kUvpX x kUvpY x kUvpZ faces.  One producer
-// warp streams each tile's boxes into a ring of kUvpStages shared-memory
-// stages (cp.async.bulk.tensor, no multicast, this GPU's own fields): pi',
-// pi'_prev, theta', theta_b and qv with one cell toward -x and -y and one
-// level below and above, and u, tu, v, tv of the tile.  Consumer thread
-// (tx, ty, tz) owns the u and v faces of cell (i0+tx, j0+ty, k0+tz):
-//   * interior faces from shared memory with uv_body's expressions;
-//   * the faces uv_body computes with the generic expressions (levels 0 and
-//     nz-1, u at j = 0, v at i = 0) from shared memory when the column has no
-//     terrain slope there (those expressions, with the same values);
-//   * every other face -- lateral edges with the radiation or periodic
-//     condition, sloped non-interior faces -- and u(nx), v(ny) by the
-//     thread of the cell beside them, with uv_body's global-memory path.
-// Every stage wait is bounded in wall time; on a timeout *err is set.
-constexpr int kUvpStages = 3;
-constexpr int kUvpThreads = kUvpX * kUvpY * kUvpZ;
-constexpr uint64_t kUvpWaitNs = 4000000000ull;
+// ------------------------------------ forward u, v in short column marches
+// A thread owns the u and v faces of KS levels of one interior (i, j): its
+// metric and its index arithmetic are worked out once, the west neighbour's
+// theta_v and pi* come from the lane beside it by shuffle (lane 0 loads
+// them), the south neighbour's from memory (lines the warp beside it has just
+// loaded), and over terrain the pi* above and below are values the march
+// holds anyway.  The faces that are not interior -- the bottom and top
+// levels, the first and last row and column -- go to blocks of their own, one
+// thread per point, on uv_body's generic path, so the march carries no edge
+// branches.  The same expressions on the same values (roundings of the
+// gradient spelled out, so that no two levels of a thread share one):
+// bit-identical.
+//
+// What bounds it: uv_body issues about 310 instructions per 32 points, of
+// which an eighth is arithmetic; the march issues about a third of that and
+// is left waiting for its loads.  KS trades instructions against resident
+// threads: one level wins on flat grids, two over terrain, and uv_body's
+// blocks on grids of a few rows, where the edge points are a third of all
+// (the tuner picks; four levels a thread were slower everywhere).  Per launch
+// (event-timed in a step, 4.7 us of event nodes included) against the better
+// block shape of uv_body: 160x160x40 FP32 16.6 against 21.6 us, FP64 27.5
+// against 31.9, 181x203x53 27.8 against 35.5, over terrain 120x90x45 16.9
+// against 21.6 and 300x200x45 49.7 against 59.3.
+constexpr int kUvmX = 32, kUvmY = 8;
 
-template <typename R>
-struct UvpLayout {
-  size_t field[UV_N];
-  size_t stage0, stage_bytes, total;
-  uint32_t tx_bytes;
-  __host__ __device__ UvpLayout(bool moist) {
-    size_t o = 0;
-    tx_bytes = 0;
-    for (int f = 0; f < UV_N; ++f) {
-      field[f] = 0;
-      if (f == UV_QV && !moist) continue;
-      int bx, by, bz;
-      uv_pipe_box(f, &bx, &by, &bz);
-      const size_t b = (size_t)bx * by * bz * sizeof(R);
-      field[f] = o;
-      o += (b + 127) / 128 * 128;
-      tx_bytes += (uint32_t)b;
-    }
-    stage_bytes = o;
-    stage0 = 128;
-    total = stage0 + (size_t)kUvpStages * stage_bytes;
-  }
-};
-
-template <typename R>
-__global__ void __launch_bounds__(kUvpThreads + 32, 1)
-    k_acoustic_uv_pipe(const __grid_constant__ PipeUvParams<R> p) {
-  extern __shared__ __align__(128) unsigned char smem_uvp[];
-  const AcouArgs<R>& a = p.a;
-  const Layout& L = a.L;
-  const bool moist = a.p.moisture != 0;
-  const UvpLayout<R> lay(moist);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_uvp);
-  uint64_t* empty = full + kUvpStages;
-  const int tid = threadIdx.x;
-  const int ntx = (L.nx + kUvpX - 1) / kUvpX, nty = (L.ny + kUvpY - 1) / kUvpY;
-  const int ntz = (L.nz + kUvpZ - 1) / kUvpZ;
-  const int ntiles = ntx * nty * ntz;
-  if (tid == 0) {
-    for (int s = 0; s < kUvpStages; ++s) {
-      tma::mbar_init(&full[s], 1);
-      tma::mbar_init(&empty[s], 1);
-    }
-    tma::fence_barrier_init();
-  }
-  __syncthreads();
-  if (tid >= kUvpThreads) {
-    // ------------------------------------------------------------ producer
-    if (tid != kUvpThreads) return;
-    int n = 0, armed[kUvpStages];
-    for (int s = 0; s < kUvpStages; ++s) armed[s] = -1;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++n) {
-      const int s = n % kUvpStages, use = n / kUvpStages;
-      if (use > 0 && !tma::mbar_wait_for(&empty[s], (use - 1) & 1, kUvpWaitNs)) {
-        atomicExch(p.err, 1u);
-        break;
-      }
-      tma::mbar_arrive_expect_tx(&full[s], lay.tx_bytes);
-      armed[s] = use;
-      unsigned char* stg = smem_uvp + lay.stage0 + (size_t)s * lay.stage_bytes;
-      const int i0 = (t % ntx) * kUvpX, j0 = (t / ntx % nty) * kUvpY, k0 = t / (ntx * nty) * kUvpZ;
-      for (int f = 0; f < UV_N; ++f) {
-        if (f == UV_QV && !moist) continue;
-        const bool halo = f <= UV_QV;
-        tma::load_3d(stg + lay.field[f], &p.map[f], i0 + kOX - (halo ? 4 : 0),
-                     j0 + kOY - (halo ? 1 : 0), k0 + kOZ - (halo ? 1 : 0), &full[s]);
-      }
-    }
-    for (int s = 0; s < kUvpStages; ++s)
-      if (armed[s] >= 0) tma::mbar_wait_for(&full[s], armed[s] & 1, kUvpWaitNs);
+// the points with a face that is not interior: levels 0 and nz - 1 whole, and
+// of the levels between them rows 0 and ny, then columns 0 and nx
+__host__ __device__ inline int uv_edge_points(const Layout& L) {
+  const int plane = (L.nx + 1) * (L.ny + 1), ring = 2 * (L.nx + 1) + 2 * (L.ny > 1 ? L.ny - 1 : 0);
+  return (L.nz > 1 ? 2 : 1) * plane + (L.nz > 2 ? L.nz - 2 : 0) * ring;
+}
+__device__ __forceinline__ void uv_edge_point(const Layout& L, int e, int* i, int* j, int* k) {
+  const int plane = (L.nx + 1) * (L.ny + 1), planes = L.nz > 1 ? 2 : 1;
+  if (e < planes * plane) {
+    *k = e < plane ? 0 : L.nz - 1;
+    const int p = e < plane ? e : e - plane;
+    *j = p / (L.nx + 1);
+    *i = p - *j * (L.nx + 1);
     return;
   }
-  // -------------------------------------------------------------- consumers
-  const int tx = tid % kUvpX, ty = tid / kUvpX % kUvpY, tz = tid / (kUvpX * kUvpY);
-  constexpr int HX = kUvpX + 4, HY = kUvpY + 1;
-  int n = 0;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++n) {
-    const int s = n % kUvpStages, use = n / kUvpStages;
-    const bool ok = tma::mbar_wait_for(&full[s], use & 1, kUvpWaitNs);
-    if (tma::named_or(1, kUvpThreads, !ok)) {
-      if (tid == 0) atomicExch(p.err, 1u);
-      break;
+  e -= planes * plane;
+  const int row = L.nx + 1, cols = L.ny > 1 ? L.ny - 1 : 0, ring = 2 * row + 2 * cols;
+  *k = 1 + e / ring;
+  const int p = e % ring;
+  if (p < 2 * row) {
+    *j = p < row ? 0 : L.ny;
+    *i = p < row ? p : p - row;
+  } else {
+    const int q = p - 2 * row;
+    *i = q < cols ? 0 : L.nx;
+    *j = 1 + (q < cols ? q : q - cols);
+  }
+}
+
+template <typename R, bool HB, bool MOIST, int KS>
+__global__ void __launch_bounds__(kUvmX * kUvmY, sizeof(R) == 4 ? 5 : 3)
+    k_acoustic_uv_march(AcouArgs<R> a, int edge_layers) {
+  const Layout& L = a.L;
+  if ((int)blockIdx.z < edge_layers) {
+    const int b = ((int)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const int e = b * (kUvmX * kUvmY) + (int)(threadIdx.y * kUvmX + threadIdx.x);
+    if (e >= uv_edge_points(L)) return;
+    int i, j, k;
+    uv_edge_point(L, e, &i, &j, &k);
+    if (j < L.ny) a.u_out[L.ati(i, j, k)] = u_face_edge(a, i, j, k);
+    if (i < L.nx) a.v_out[L.ati(i, j, k)] = v_face_edge(a, i, j, k);
+    return;
+  }
+  const int lane = threadIdx.x;
+  const int j = 1 + (int)blockIdx.y * kUvmY + (int)threadIdx.y;
+  const int k0 = 1 + ((int)blockIdx.z - edge_layers) * KS;
+  if (j >= L.ny) return;  // whole warps
+  const int iq = 1 + (int)blockIdx.x * kUvmX + lane;
+  const bool mine = iq < L.nx;
+  const int i = mine ? iq : L.nx - 1;  // lanes past the row repeat its last point
+  const int sy = L.px, pl = L.planei();
+  const int c2 = L.at2i(i, j);
+  const R hxu = a.m.hx_u[c2], hyv = a.m.hy_v[c2];
+  const R m0 = a.m.mapf[c2];
+  const R mfu = (R)0.5 * (a.m.mapf[c2 - 1] + m0);
+  const R mfv = (R)0.5 * (a.m.mapf[c2 - sy] + m0);
+  const bool hills = __any_sync(0xffffffffu, hxu != (R)0 || hyv != (R)0);
+  const R smdiv = a.p.acoustic_smdiv, dtau = a.dtau;
+  const int top = L.nz - 2;  // the last interior level
+  const int c = L.ati(i, j, k0);
+
+  R tv0[KS], tvx[KS], tvy[KS], uin[KS], vin[KS], tun[KS], tvn[KS];
+  R ps0[KS + 2], psx[KS + 2], psy[KS + 2];  // levels k0 - 1 .. k0 + KS
+  auto pistar_of = [&](int cc) {
+    const R cur = a.pi_cur[cc];
+    return cur + smdiv * (cur - a.pi_prev[cc]);
+  };
+#pragma unroll
+  for (int q = 0; q < KS; ++q) {
+    // levels past the last interior one repeat it
+    const int d = (k0 + q <= top ? q : top - k0) * pl;
+    const int kk = L.at1(k0 + q <= top ? k0 + q : top);
+    const int cc = c + d;
+    auto thv = [&](int x) {
+      R t = (HB ? a.b.lvl[BL_THB * L.pz + kk] : a.b.thb[x]) + a.th_in[x];
+      if (MOIST) t *= (R)1 + Phys<R>::eps61 * a.qv[x];
+      return t;
+    };
+    ps0[q + 1] = pistar_of(cc);
+    tv0[q] = thv(cc);
+    psy[q + 1] = pistar_of(cc - sy);
+    tvy[q] = thv(cc - sy);
+    psx[q + 1] = tvx[q] = 0;
+    if (lane == 0) {
+      psx[q + 1] = pistar_of(cc - 1);
+      tvx[q] = thv(cc - 1);
     }
-    const unsigned char* stg = smem_uvp + lay.stage0 + (size_t)s * lay.stage_bytes;
-    auto fld = [&](int f) { return reinterpret_cast<const R*>(stg + lay.field[f]); };
-    const R* sPI = fld(UV_PI);
-    const R* sPP = fld(UV_PIP);
-    const R* sTH = fld(UV_TH);
-    const R* sTB = fld(UV_THB);
-    const R* sQV = fld(UV_QV);
-    const int i0 = (t % ntx) * kUvpX, j0 = (t / ntx % nty) * kUvpY, k0 = t / (ntx * nty) * kUvpZ;
-    const int i = i0 + tx, j = j0 + ty, k = k0 + tz;
-    // halo-box index of cell (i + dx, j + dy, k + dz)
-    auto hix = [&](int dx, int dy, int dz) { return ((tz + 1 + dz) * HY + (ty + 1 + dy)) * HX + tx + 4 + dx; };
-    auto thv = [&](int h) {  // theta_v_at from shared memory
-      R tv = sTB[h] + sTH[h];
-      if (moist) tv *= (R)1 + Phys<R>::eps61 * sQV[h];
-      return tv;
-    };
-    auto pst = [&](int h) {  // pistar_at from shared memory
-      R cur = sPI[h];
-      return cur + a.p.acoustic_smdiv * (cur - sPP[h]);
-    };
-    R uo = 0, vo = 0;
-    bool u_done = false, v_done = false;
-    const bool cell = i < L.nx && j < L.ny && k < L.nz;
-    if (cell) {
-      const int kk = L.at1(k);
-      const int c2 = L.at2i(i, j);
-      const int t0 = (tz * kUvpY + ty) * kUvpX + tx;  // tile-box index
-      const int h0 = hix(0, 0, 0);
-      const R tv0 = thv(h0), ps0 = pst(h0);
-      if (uv_interior<R>(L, i, j, k)) {
-        const R tvx = thv(h0 - 1), psx = pst(h0 - 1);
-        const R tvy = thv(h0 - HX), psy = pst(h0 - HX);
-        uo = u_interior_core(a, c2, kk, tv0, tvx, ps0, psx, fld(UV_U)[t0], fld(UV_TU)[t0], [&](R* q) {
-          q[0] = pst(hix(-1, 0, 1));
-          q[1] = pst(hix(-1, 0, -1));
-          q[2] = pst(hix(0, 0, 1));
-          q[3] = pst(hix(0, 0, -1));
-        });
-        vo = v_interior_core(a, c2, kk, tv0, tvy, ps0, psy, fld(UV_V)[t0], fld(UV_TV)[t0], [&](R* q) {
-          q[0] = pst(hix(0, -1, 1));
-          q[1] = pst(hix(0, -1, -1));
-          q[2] = pst(hix(0, 0, 1));
-          q[3] = pst(hix(0, 0, -1));
-        });
-        u_done = v_done = true;
-      } else {
-        // uv_body's generic expressions (u_forward / v_forward) where they
-        // read only this tile's cells and no terrain term
-        if (i >= 1 && a.m.hx_u[c2] * ((R)1 - a.m.zeta_c[kk] / a.m.zt) == (R)0) {
-          R thbu = (R)0.5 * (thv(h0 - 1) + tv0);
-          R mu = (R)0.5 * (a.m.mapf[c2 - 1] + a.m.mapf[c2]);
-          R grad = (ps0 - pst(h0 - 1)) / a.dx;
-          uo = fld(UV_U)[t0] + a.dtau * (-Phys<R>::cp * thbu * mu * grad + fld(UV_TU)[t0]);
-          u_done = true;
-        }
-        if (j >= 1 && a.m.hy_v[c2] * ((R)1 - a.m.zeta_c[kk] / a.m.zt) == (R)0) {
-          R thbv = (R)0.5 * (thv(h0 - HX) + tv0);
-          R mv = (R)0.5 * (a.m.mapf[c2 - L.px] + a.m.mapf[c2]);
-          R grad = (ps0 - pst(h0 - HX)) / a.dy;
-          vo = fld(UV_V)[t0] + a.dtau * (-Phys<R>::cp * thbv * mv * grad + fld(UV_TV)[t0]);
-          v_done = true;
-        }
+    uin[q] = a.u_in[cc];
+    vin[q] = a.v_in[cc];
+    tun[q] = a.tu[cc];
+    tvn[q] = a.tv[cc];
+  }
+  ps0[0] = ps0[KS + 1] = psx[0] = psx[KS + 1] = psy[0] = psy[KS + 1] = 0;
+  R jfu = 1, jfv = 1;
+  if (hills) {
+    const R j0 = a.m.jac[c2];
+    jfu = (R)0.5 * (a.m.jac[c2 - 1] + j0);
+    jfv = (R)0.5 * (a.m.jac[c2 - sy] + j0);
+    const int ce = c + (k0 + KS <= top + 1 ? KS : top + 1 - k0) * pl;
+    ps0[0] = pistar_of(c - pl);
+    psy[0] = pistar_of(c - pl - sy);
+    ps0[KS + 1] = pistar_of(ce);
+    psy[KS + 1] = pistar_of(ce - sy);
+    if (lane == 0) {
+      psx[0] = pistar_of(c - pl - 1);
+      psx[KS + 1] = pistar_of(ce - 1);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < KS + 2; ++q) {
+    const R x = __shfl_up_sync(0xffffffffu, ps0[q], 1);
+    if (lane > 0) psx[q] = x;
+  }
+#pragma unroll
+  for (int q = 0; q < KS; ++q) {
+    const R x = __shfl_up_sync(0xffffffffu, tv0[q], 1);
+    if (lane > 0) tvx[q] = x;
+  }
+  if (!mine) return;
+#pragma unroll
+  for (int q = 0; q < KS; ++q) {
+    if (k0 + q > top) break;
+    const int kk = L.at1(k0 + q);
+    const int cc = c + q * pl;
+    {
+      R thb_f = (R)0.5 * (tvx[q] + tv0[q]);
+      R mf = mfu;
+      R grad = mul_rn(ps0[q + 1] - psx[q + 1], a.co.inv_dx);
+      const R slope = hxu * a.co.fac_c[kk];
+      if (slope != (R)0) {
+        // the level above the segment's last interior one is in its last slot
+        const R x2 = k0 + q == top ? psx[KS + 1] : psx[q + 2], p2 = k0 + q == top ? ps0[KS + 1] : ps0[q + 2];
+        R dpdz = (R)0.5 * ((x2 - psx[q]) + (p2 - ps0[q])) * a.co.inv_dzc2[kk];
+        grad = fma_rn(-(slope / jfu), dpdz, grad);
       }
+      a.u_out[cc] = uin[q] + dtau * fma_rn(-Phys<R>::cp * thb_f * mf, grad, tun[q]);
     }
-    // every input of the tile has been read from shared memory: the producer
-    // may refill the stage
-    tma::named_sync(1, kUvpThreads);
-    if (tid == 0) tma::mbar_arrive(&empty[s]);
-    if (cell) {
-      const int c = L.ati(i, j, k);
-      a.u_out[c] = u_done ? uo : u_face_edge(a, i, j, k);
-      a.v_out[c] = v_done ? vo : v_face_edge(a, i, j, k);
-      if (i == L.nx - 1) a.u_out[L.ati(L.nx, j, k)] = u_face_edge(a, L.nx, j, k);
-      if (j == L.ny - 1) a.v_out[L.ati(i, L.ny, k)] = v_face_edge(a, i, L.ny, k);
+    {
+      R thb_f = (R)0.5 * (tvy[q] + tv0[q]);
+      R mf = mfv;
+      R grad = mul_rn(ps0[q + 1] - psy[q + 1], a.co.inv_dy);
+      const R slope = hyv * a.co.fac_c[kk];
+      if (slope != (R)0) {
+        const R y2 = k0 + q == top ? psy[KS + 1] : psy[q + 2], p2 = k0 + q == top ? ps0[KS + 1] : ps0[q + 2];
+        R dpdz = (R)0.5 * ((y2 - psy[q]) + (p2 - ps0[q])) * a.co.inv_dzc2[kk];
+        grad = fma_rn(-(slope / jfv), dpdz, grad);
+      }
+      a.v_out[cc] = vin[q] + dtau * fma_rn(-Phys<R>::cp * thb_f * mf, grad, tvn[q]);
     }
   }
 }
@@ -1062,10 +1059,36 @@ static void launch_uv_shape(const AcouArgs<R>& a, cudaStream_t st) {
   else k_acoustic_uv<R, false, S><<<g, t, 0, st>>>(a);
 }
 
+template <typename R, int KS>
+static void launch_uv_march(const AcouArgs<R>& a, cudaStream_t st) {
+  const Layout& L = a.L;
+  auto blocks = [](int n, int b) { return n > 0 ? (n + b - 1) / b : 0; };
+  dim3 g(blocks(L.nx - 1, kUvmX), blocks(L.ny - 1, kUvmY), blocks(L.nz - 2, KS));
+  const bool inner = g.x && g.y && g.z;
+  const int edge = blocks(uv_edge_points(L), kUvmX * kUvmY);
+  int layers;
+  if (inner) {
+    layers = blocks(edge, (int)(g.x * g.y));
+    g.z += layers;
+  } else {  // a grid without an interior point
+    g = dim3(edge, 1, 1);
+    layers = 1;
+  }
+  const dim3 t(kUvmX, kUvmY);
+  if (a.b.lvl && a.p.moisture) k_acoustic_uv_march<R, true, true, KS><<<g, t, 0, st>>>(a, layers);
+  else if (a.b.lvl) k_acoustic_uv_march<R, true, false, KS><<<g, t, 0, st>>>(a, layers);
+  else if (a.p.moisture) k_acoustic_uv_march<R, false, true, KS><<<g, t, 0, st>>>(a, layers);
+  else k_acoustic_uv_march<R, false, false, KS><<<g, t, 0, st>>>(a, layers);
+}
+
 template <typename R>
 void launch_acoustic_uv(const AcouArgs<R>& a, cudaStream_t st, int shape) {
-  if (shape == 1) launch_uv_shape<R, 1>(a, st);
-  else launch_uv_shape<R, 0>(a, st);
+  switch (shape) {
+    case 1: launch_uv_march<R, 2>(a, st); break;
+    case 2: launch_uv_shape<R, 1>(a, st); break;
+    case 3: launch_uv_march<R, 1>(a, st); break;
+    default: launch_uv_shape<R, 0>(a, st); break;
+  }
 }
 
 template <typename R>
@@ -1298,46 +1321,7 @@ int occupancy_column(int shape, int nz_max) {
   return e == cudaSuccess && n > 0 ? n : 1;
 }
 
-template <typename R>
-int prepare_acoustic_uv_pipe() {
-  const size_t sm = UvpLayout<R>(true).total;
-  if (sm > 227 * 1024) return 2;
-  return raise_smem_limit(k_acoustic_uv_pipe<R>, sm) == cudaSuccess ? 0 : 1;
-}
-
-template <typename R>
-int launch_acoustic_uv_pipe(const PipeUvParams<R>& p, cudaStream_t st) {
-  const size_t sm = UvpLayout<R>(p.a.p.moisture != 0).total;
-  if (sm > 227 * 1024) return 2;
-  static std::mutex mu;
-  static std::map<std::pair<int, size_t>, int> limit;  // (device, smem) -> resident CTAs
-  int dev = 0, lim = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 2;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = limit.find(std::make_pair(dev, sm));
-    if (it != limit.end()) {
-      lim = it->second;
-    } else {
-      int sms = 0, occ = 0;
-      if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_acoustic_uv_pipe<R>, kUvpThreads + 32,
-                                                        sm) != cudaSuccess)
-        return 2;
-      lim = limit[std::make_pair(dev, sm)] = sms * occ;
-    }
-  }
-  if (lim <= 0) return 2;
-  const Layout& L = p.a.L;
-  const int ntiles = ((L.nx + kUvpX - 1) / kUvpX) * ((L.ny + kUvpY - 1) / kUvpY) *
-                     ((L.nz + kUvpZ - 1) / kUvpZ);
-  k_acoustic_uv_pipe<R><<<ntiles < lim ? ntiles : lim, kUvpThreads + 32, sm, st>>>(p);
-  return 0;
-}
-
 #define WFE_INST(R)                                                                            \
-  template int prepare_acoustic_uv_pipe<R>();                                                  \
-  template int launch_acoustic_uv_pipe<R>(const PipeUvParams<R>&, cudaStream_t);               \
   template dim3 grid_uv<R>(const Layout&);                                                     \
   template dim3 grid_uv_fwd<R>(const Layout&);                                                 \
   template dim3 grid_column<R>(const Layout&, int);                                            \

@@ -331,8 +331,8 @@ template <typename R>
 void launch_acoustic_coef(const Layout& L, const DBase<R>& b, const DMetric<R>& m, R* scratch,
                           R* rtjx, R* rtjy, R* kt3, R* aw, cudaStream_t st);
 template <typename R>
-// shape 0: 16 x 16 x 1 face tiles, 1: 32 x 2 x 4 (grids of few rows); the
-// same values either way
+// shape 0: 16 x 16 x 1 face tiles, 2: 32 x 2 x 4 (grids of few rows), 1 and
+// 3: column marches of two levels and of one; the same values
 void launch_acoustic_uv(const AcouArgs<R>& a, cudaStream_t st, int shape = 0);
 // The column's input fields in the order of the pipelined kernels' tensor maps:
 enum {
@@ -381,32 +381,6 @@ template <typename R>
 size_t acoustic_pipe_pcr_smem(int shape, int nz, bool moist, bool tpi, bool prof = false);
 template <typename R>
 int launch_acoustic_column_pipe_pcr(const PipeColParams<R>& p, int shape, cudaStream_t st);
-// Persistent, pipelined forward u, v kernel (dyn_acou_pipe.cu): tiles of
-// kUvpX x kUvpY x kUvpZ faces; a producer warp streams each tile's boxes (the
-// cell fields with a one-cell halo toward -x, -y and +-z, the face fields
-// without) into a ring of shared-memory stages; interior faces are computed
-// from shared memory with the u, v kernel's expressions (bit-identical),
-// the lateral edge faces (radiation or periodic) by its global-memory path.
-enum { UV_PI = 0, UV_PIP, UV_TH, UV_THB, UV_QV, UV_U, UV_TU, UV_V, UV_TV, UV_N };
-constexpr int kUvpX = 32, kUvpY = 4, kUvpZ = 4;
-// box extents of map f
-WFE_HD void uv_pipe_box(int f, int* bx, int* by, int* bz) {
-  const bool halo = f <= UV_QV;
-  *bx = halo ? kUvpX + 4 : kUvpX;
-  *by = halo ? kUvpY + 1 : kUvpY;
-  *bz = halo ? kUvpZ + 2 : kUvpZ;
-}
-template <typename R>
-struct PipeUvParams {
-  AcouArgs<R> a;
-  unsigned* err;
-  CUtensorMap map[UV_N];
-};
-template <typename R>
-int prepare_acoustic_uv_pipe();
-// Returns 0 ok, 2 not usable
-template <typename R>
-int launch_acoustic_uv_pipe(const PipeUvParams<R>& p, cudaStream_t st);
 // shape: tile-shape index (columns x level lanes) in [0, acoustic_column_shapes());
 // one that does not fit the column depth falls back to the first that does
 template <typename R>

@@ -36,6 +36,9 @@
 
 namespace wfe {
 
+// forward u, v variants (Tune::uv_variant)
+constexpr int kUvVariants = 4;
+
 // Kernel variants picked by the autotuner.  Every variant computes the same
 // values with the same arithmetic; only launch shapes differ.
 struct Tune {
@@ -44,8 +47,8 @@ struct Tune {
   int column_cx = 0;     // acoustic column tile shape index (launch_acoustic_column)
   int persist = 0;       // ensembles: 0 one block per work item, 1 persistent grid, 2 members' own
                          // graphs on concurrent streams, 3 members' own graphs one after another
-  int uv_variant = 0;    // forward u, v: 0 thread per face pair in 16 x 16 x 1 blocks, 1 persistent
-                         // pipelined tiles, 2 thread per face pair in 32 x 2 x 4 blocks
+  int uv_variant = 0;    // forward u, v: 0 thread per face pair in 16 x 16 x 1 blocks, 2 in
+                         // 32 x 2 x 4 blocks, 1 and 3 column marches of two levels and of one
   bool done = false;
 };
 
@@ -138,7 +141,6 @@ class ModelT final : public Model {
     fused_ok_ = prepare_acoustic_fused<R>(g_.nz) == 0;
     reg_ok_ = prepare_acoustic_reg<R>(g_.nz) == 0;
     pipe_ok_ = tensor_map_encoder() && prepare_acoustic_pipe<R>(g_.nz) == 0;
-    uvp_ok_ = tensor_map_encoder() && prepare_acoustic_uv_pipe<R>() == 0;
     tend_tma_ok_ = tensor_map_encoder() && tend_scal_tma_smem<R>() <= 227 * 1024 &&
                    prepare_tend_scal_tma<R>() == 0;
     CK(cudaMalloc(&tma_err_, sizeof(unsigned)));
@@ -848,7 +850,7 @@ class ModelT final : public Model {
     std::string name = prop.name;
     for (char& ch : name)
       if (ch == ' ') ch = '_';
-    k << "v10|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
+    k << "v11|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
       << dp_.moisture << "pd" << dp_.pd_moist << "b" << bdy_on_ << "d" << (dp_.diff_K > 0) << "x"
       << (pcr_allowed() ? 0 : 1);
     return k.str();
@@ -897,8 +899,8 @@ class ModelT final : public Model {
   // column kernel in six shapes, 16..18 the parallel-solve column kernel and
   // 19..22 its pipelined form, both equal to the others up to rounding),
   // WFE_UV_VARIANT=<n> the forward u, v kernel (0
-  // thread per face pair in 16 x 16 x 1 blocks, 1 persistent pipelined tiles,
-  // 2 thread per face pair in 32 x 2 x 4 blocks) and WFE_TEND_VARIANT=<n>
+  // thread per face pair in 16 x 16 x 1 blocks, 2 in 32 x 2 x 4 blocks, 1 and
+  // 3 column marches of two levels and of one) and WFE_TEND_VARIANT=<n>
   // the tendency variant (0 fused, 1 split, 2 momentum + TMA-staged scalars,
   // 3 fused with two cells per thread)
   // after tuning, for tests and experiments
@@ -915,7 +917,7 @@ class ModelT final : public Model {
     const char* uvv = std::getenv("WFE_UV_VARIANT");
     if (first && uvv && *uvv) {
       const int v = std::atoi(uvv);
-      if (v == 0 || (v == 1 && uvp_ok_) || v == 2) tune_.uv_variant = v;
+      if (v >= 0 && v < kUvVariants) tune_.uv_variant = v;
     }
     const char* tv = std::getenv("WFE_TEND_VARIANT");
     if (first && tv && *tv) {
@@ -957,9 +959,8 @@ class ModelT final : public Model {
     best = 1e30f;
     const int ns = hp_.acoustic_ns > 1 ? hp_.acoustic_ns : 1;
     // 0 and 2: one thread per face pair in square and slab-shaped blocks;
-    // 1: the persistent pipelined tiles
-    for (int v = 0; v < 3; ++v) {
-      if (v == 1 && !uvp_ok_) continue;
+    // 1 and 3: short column marches
+    for (int v = 0; v < kUvVariants; ++v) {
       float ms;
       tune_.uv_variant = v;
       if (time_ms([&] { return acoustic(N, X, (R)dt / (R)ns, 1, false); }, &ms)) return 1;
@@ -1131,15 +1132,7 @@ class ModelT final : public Model {
 
   // The tuned forward u, v launch of one substep.
   int uv_launch(const AcouArgs<R>& a) {
-    int rc = 0;
-    if (uvp_ok_ && tune_.uv_variant == 1) {
-      PipeUvParams<R> up;
-      if (uv_pipe_params(a, &up)) return 1;
-      launch("acoustic_uv", [&] { rc = launch_acoustic_uv_pipe<R>(up, st_); });
-      if (rc) return fail("pipelined u, v launch");
-    } else {
-      launch("acoustic_uv", [&] { launch_acoustic_uv<R>(a, st_, tune_.uv_variant == 2 ? 1 : 0); });
-    }
+    launch("acoustic_uv", [&] { launch_acoustic_uv<R>(a, st_, tune_.uv_variant); });
     return 0;
   }
 
@@ -1281,22 +1274,6 @@ class ModelT final : public Model {
       const CUtensorMap* x = tmap3(q[f], kTtX + 8, kTtY + 6, kTtZ + 6);
       if (!x) return 1;
       tp->q[f] = *x;
-    }
-    return 0;
-  }
-
-  int uv_pipe_params(const AcouArgs<R>& a, PipeUvParams<R>* up) {
-    std::memset(static_cast<void*>(up), 0, sizeof(*up));
-    up->a = a;
-    up->err = tma_err_;
-    const R* src[UV_N] = {a.pi_cur, a.pi_prev, a.th_in, a.b.thb, a.qv, a.u_in, a.tu, a.v_in, a.tv};
-    for (int f = 0; f < UV_N; ++f) {
-      if (f == UV_QV && !a.p.moisture) continue;
-      int bx, by, bz;
-      uv_pipe_box(f, &bx, &by, &bz);
-      const CUtensorMap* m = tmap3(src[f], bx, by, bz);
-      if (!m) return 1;
-      up->map[f] = *m;
     }
     return 0;
   }
@@ -1487,6 +1464,7 @@ class ModelT final : public Model {
     const int hw = (int)std::thread::hardware_concurrency();
     t = std::min({t, 4, hw > 0 ? hw : 1, n});
     std::vector<std::thread> th;
+    th.reserve(4);
     int done = 0;  // levels handed out
     for (int q = 1; q < t; ++q) {
       const int k0 = done, k1 = (int)((long)n * q / t);
@@ -1660,7 +1638,6 @@ class ModelT final : public Model {
   bool fused_ok_ = false;            // fused substep kernels prepared
   bool reg_ok_ = false;              // register-held column variants usable
   bool pipe_ok_ = false;             // pipelined column kernels prepared
-  bool uvp_ok_ = false;              // pipelined u, v kernel prepared
   bool tend_tma_ok_ = false;         // TMA-staged scalar tendencies usable
   R* lvl_tab_ = nullptr;             // the column coefficients' level tables (PF_*), or null
   unsigned* tma_err_ = nullptr;      // set by a TMA tile load that timed out
