@@ -108,6 +108,7 @@ KERNEL_FIELDS = {
     "tendencies": 22,
     "mass_flux": 8,     # u v w rho_b rho_b^w -> mfx mfy mfz
     "kessler": 12,      # theta' pi' qv qc qr theta_b pi_b rho_b -> theta' qv qc qr
+    "moist_terms": 6,   # qv qc qr qv_b -> the column's two moisture terms
     "pd_ratio": 8,
     "fill_ghosts": 0,   # surface-area only
 }
@@ -732,6 +733,12 @@ def main():
             if kname in kf and (kname != "kessler" or moist):
                 kf = dict(kf, **{kname: kf[kname] - nf})
                 step_fields -= nf * kt.get(kname, (0.0, 0))[1]
+    if "moist_terms" in kt:
+        # the column reads the step's two moisture terms instead of qv, qc, qr
+        # (and qv_b, unless that comes from its table)
+        less = 1 if tables else 2
+        kf = dict(kf, acoustic_column=kf["acoustic_column"] - less)
+        step_fields += kf["moist_terms"] - less * kt.get("acoustic_column", (0.0, 0))[1]
     alg_bytes = kf.get(dom_name, 0) * 4 * cells
     hbm, peak_kind = peaks()
     achieved = alg_bytes / (avg_ms / 1000.0) / 1e9

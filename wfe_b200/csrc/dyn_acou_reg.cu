@@ -25,7 +25,8 @@
 // recomputed edges, and a producer warp's ring of bulk loads in front of the
 // same sweep: 160x160x40 flat FP32 29.7 against 48.3 us, FP64 59.6 against
 // 84.4, 181x203x53 60 against 85.6, 300x200x45 over terrain 121-127 against
-// 142, 512x4x64 13.2 against 16.8.
+// 142, 512x4x64 13.2 against 16.8.  With the moisture as the step's two terms
+// (MOIST_TERMS) instead of four fields: 27.7, 49.6, 54.6 and 115.7 us.
 #include <cuda_runtime.h>
 
 #include "core.cuh"
@@ -35,6 +36,27 @@
 namespace wfe {
 
 namespace {
+
+// where a column's moisture comes from: nowhere (dry), qv, qc, qr and qv_b, or
+// the two terms they make on w levels, the same in every substep of a step
+// (AcouArgs::mq, mb)
+enum { MOIST_NONE = 0, MOIST_FIELDS = 1, MOIST_TERMS = 2 };
+
+// The two moisture terms of the inner w levels from the time-n species, which
+// no substep changes: the factor of theta_v^w and the moist part of the
+// buoyancy, rounded as the column kernels round them.
+template <typename R>
+__global__ void __launch_bounds__(256) k_moist_terms(Layout L, const R* __restrict__ qv, const R* __restrict__ qc,
+                                                     const R* __restrict__ qr, const R* __restrict__ qvb,
+                                                     R* __restrict__ mq, R* __restrict__ mb) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, k = 1 + blockIdx.z;
+  if (i >= L.nx || j >= L.ny) return;
+  const int c = L.ati(i, j, k), cm = c - L.planei();
+  mq[c] = (R)1 + Phys<R>::eps61 * (R)0.5 * (qv[cm] + qv[c]);
+  const R dqv = (R)0.5 * (qv[cm] + qv[c]) - (R)0.5 * (qvb[cm] + qvb[c]);
+  const R qcr = (R)0.5 * (qc[cm] + qc[c]) + (R)0.5 * (qr[cm] + qr[c]);
+  mb[c] = fma_rn(Phys<R>::eps61, dqv, -qcr);
+}
 
 // shared values per (lane, column): the chunk edges
 enum { XU_SU = 0, XU_SV, XU_AV, XU_PI, XU_TH, XU_QV, XU_QC, XU_QR, XU_QVB, XU_P, XU_E, XD_AV, XD_W, XD_SV, X_N };
@@ -47,7 +69,7 @@ __device__ __forceinline__ R flux_diff(R a, R b, R c, R d) {
   return fma_rn(a, b, -mul_rn(c, d));
 }
 
-template <typename R, int CX, int KCH, bool PROF, bool MOIST, bool TPI>
+template <typename R, int CX, int KCH, bool PROF, int MOIST, bool TPI>
 __device__ __forceinline__ void column_reg_body(const AcouArgs<R>& a, const R* __restrict__ prof, R* smem) {
   const Layout& L = a.L;
   const int nz = L.nz;
@@ -108,11 +130,14 @@ __device__ __forceinline__ void column_reg_body(const AcouArgs<R>& a, const R* _
     pi[q] = a.pi_cur[c];
     th[q] = a.th_in[c];
     tw[q] = a.tw[c];
-    if (MOIST) {
+    if (MOIST == MOIST_FIELDS) {
       qv[q] = a.qv[c];
       qc[q] = a.qc[c];
       qr[q] = a.qr[c];
       qvb[q] = PROF ? prof[PF_QVB * n1 + k] : a.b.qvb[c];
+    } else if (MOIST == MOIST_TERMS) {
+      qv[q] = a.mq[c];
+      qc[q] = a.mb[c];
     }
     w[q] = a.w_in[c0 + (klo + q < nz ? klo + q : nz) * pl];
     if (klo + q == 0 || klo + q >= nz) av[q] = 0;
@@ -131,7 +156,7 @@ __device__ __forceinline__ void column_reg_body(const AcouArgs<R>& a, const R* _
   EX(XU_TH, lane) = th[T];
   EX(XD_AV, lane) = av[0];
   EX(XD_W, lane) = w[0];
-  if (MOIST) {
+  if (MOIST == MOIST_FIELDS) {
     EX(XU_QV, lane) = qv[T];
     EX(XU_QC, lane) = qc[T];
     EX(XU_QR, lane) = qr[T];
@@ -195,16 +220,18 @@ __device__ __forceinline__ void column_reg_body(const AcouArgs<R>& a, const R* _
       const R pim = q ? pi[p] : EX(XU_PI, lane - 1);
       const R avm = q ? av[p] : EX(XU_AV, lane - 1);
       R qvm = 0;
-      if (MOIST) qvm = q ? qv[p] : EX(XU_QV, lane - 1);
+      if (MOIST == MOIST_FIELDS) qvm = q ? qv[p] : EX(XU_QV, lane - 1);
       const R iJdz = invJ * idzw[q];
       R thvw = thbw[q] + (R)0.5 * (thm + thc);
-      if (MOIST) thvw *= (R)1 + Phys<R>::eps61 * (R)0.5 * (qvm + qv[q]);
+      if (MOIST == MOIST_FIELDS) thvw *= (R)1 + Phys<R>::eps61 * (R)0.5 * (qvm + qv[q]);
+      if (MOIST == MOIST_TERMS) thvw *= qv[q];
       R G = dtau * Phys<R>::cp * thvw * c1 * iJdz;
       SQ(sA, k) = -G * Em * avm;
       SQ(sB, k) = (R)1 + G * av[q] * (Ek + Em);
       SQ(sC, k) = -G * Ek * av[q + 1];
       R buoy = Phys<R>::grav * (R)0.5 * (thm + thc) / thbw[q];
-      if (MOIST) {
+      if (MOIST == MOIST_TERMS) buoy = fma_rn(Phys<R>::grav, qc[q], buoy);
+      if (MOIST == MOIST_FIELDS) {
         const R qcm = q ? qc[p] : EX(XU_QC, lane - 1), qrm = q ? qr[p] : EX(XU_QR, lane - 1);
         const R qbm = q ? qvb[p] : EX(XU_QVB, lane - 1);
         R dqv = (R)0.5 * (qvm + qv[q]) - (R)0.5 * (qbm + qvb[q]);
@@ -304,7 +331,7 @@ __device__ __forceinline__ void column_reg_body(const AcouArgs<R>& a, const R* _
 #undef SQ
 }
 
-template <typename R, int CX, int KCH, int REGS, bool PROF, bool MOIST, bool TPI>
+template <typename R, int CX, int KCH, int REGS, bool PROF, int MOIST, bool TPI>
 __global__ void __maxnreg__(REGS) k_acoustic_column_reg(AcouArgs<R> a, const R* __restrict__ prof) {
   extern __shared__ __align__(16) unsigned char smem_reg[];
   column_reg_body<R, CX, KCH, PROF, MOIST, TPI>(a, prof, reinterpret_cast<R*>(smem_reg));
@@ -330,25 +357,24 @@ size_t reg_smem(int nz, int s) {
   return ((size_t)X_N * lanes(nz, kShapes[s].kch) + (size_t)4 * (nz + 1)) * kShapes[s].cx * sizeof(R);
 }
 
-// the four forms of a shape: dry or moist, with and without the slow pi'
-// tendency (only operator calls and relaxed runs have one); with tables
-// there is none
-template <typename R, int S, class F>
-void with_kernel(bool prof, bool moist, bool tpi, F&& f) {
+// the forms of a shape: dry, moist from the fields or from the step's terms,
+// with and without the slow pi' tendency (only operator calls and relaxed
+// runs have one; with it the tables are not used)
+template <typename R, int S, bool PROF, bool TPI, class F>
+void with_moisture(int moist, F&& f) {
   constexpr int CX = kShapes[S].cx, KCH = kShapes[S].kch, G = regs_of<R>(S);
-  if (prof && !tpi) {
-    if (moist) f(k_acoustic_column_reg<R, CX, KCH, G, true, true, false>);
-    else f(k_acoustic_column_reg<R, CX, KCH, G, true, false, false>);
-  } else if (tpi) {
-    if (moist) f(k_acoustic_column_reg<R, CX, KCH, G, false, true, true>);
-    else f(k_acoustic_column_reg<R, CX, KCH, G, false, false, true>);
-  } else {
-    if (moist) f(k_acoustic_column_reg<R, CX, KCH, G, false, true, false>);
-    else f(k_acoustic_column_reg<R, CX, KCH, G, false, false, false>);
-  }
+  if (moist == MOIST_TERMS) f(k_acoustic_column_reg<R, CX, KCH, G, PROF, MOIST_TERMS, TPI>);
+  else if (moist == MOIST_FIELDS) f(k_acoustic_column_reg<R, CX, KCH, G, PROF, MOIST_FIELDS, TPI>);
+  else f(k_acoustic_column_reg<R, CX, KCH, G, PROF, MOIST_NONE, TPI>);
+}
+template <typename R, int S, class F>
+void with_kernel(bool prof, int moist, bool tpi, F&& f) {
+  if (tpi) with_moisture<R, S, false, true>(moist, f);
+  else if (prof) with_moisture<R, S, true, false>(moist, f);
+  else with_moisture<R, S, false, false>(moist, f);
 }
 template <typename R, class F>
-void for_shape(int s, bool prof, bool moist, bool tpi, F&& f) {
+void for_shape(int s, bool prof, int moist, bool tpi, F&& f) {
   switch (s) {
     case 0: with_kernel<R, 0>(prof, moist, tpi, f); break;
     case 1: with_kernel<R, 1>(prof, moist, tpi, f); break;
@@ -364,6 +390,14 @@ void for_shape(int s, bool prof, bool moist, bool tpi, F&& f) {
 int acoustic_reg_shapes() { return kNumShapes; }
 
 template <typename R>
+void launch_moist_terms(const Layout& L, const DBase<R>& b, const R* qv, const R* qc, const R* qr, R* mq, R* mb,
+                        cudaStream_t st) {
+  if (L.nz < 2) return;
+  k_moist_terms<R><<<dim3((L.nx + 31) / 32, (L.ny + 7) / 8, L.nz - 1), dim3(32, 8), 0, st>>>(L, qv, qc, qr, b.qvb,
+                                                                                            mq, mb);
+}
+
+template <typename R>
 bool acoustic_reg_fits(int nz, int s) {
   if (s < 0 || s >= kNumShapes || nz < 2) return false;
   const int threads = kShapes[s].cx * lanes(nz, kShapes[s].kch), warps = (threads + 31) / 32;
@@ -376,8 +410,8 @@ int prepare_acoustic_reg(int nz) {
   int rc = 0;
   for (int s = 0; s < kNumShapes; ++s) {
     if (!acoustic_reg_fits<R>(nz, s)) continue;
-    for (int p = 0; p < 8; ++p)
-      for_shape<R>(s, p & 1, p & 2, p & 4, [&](auto* k) { rc |= raise_smem_limit(k, reg_smem<R>(nz, s)) != cudaSuccess; });
+    for (int p = 0; p < 12; ++p)
+      for_shape<R>(s, p & 1, p / 4, p & 2, [&](auto* k) { rc |= raise_smem_limit(k, reg_smem<R>(nz, s)) != cudaSuccess; });
   }
   return rc;
 }
@@ -387,13 +421,16 @@ int launch_acoustic_column_reg(const AcouArgs<R>& a, const R* prof, int s, cudaS
   const int nz = a.L.nz;
   if (!acoustic_reg_fits<R>(nz, s)) return 2;
   const dim3 grd((a.L.nx + kShapes[s].cx - 1) / kShapes[s].cx, a.L.ny), blk(kShapes[s].cx, lanes(nz, kShapes[s].kch));
-  for_shape<R>(s, prof != nullptr, a.p.moisture != 0, a.tpi != nullptr, [&](auto* k) { k<<<grd, blk, reg_smem<R>(nz, s), st>>>(a, prof); });
+  const int moist = !a.p.moisture ? MOIST_NONE : a.mq ? MOIST_TERMS : MOIST_FIELDS;
+  for_shape<R>(s, prof != nullptr, moist, a.tpi != nullptr, [&](auto* k) { k<<<grd, blk, reg_smem<R>(nz, s), st>>>(a, prof); });
   return 0;
 }
 
 #define WFE_INST(R)                                       \
   template bool acoustic_reg_fits<R>(int, int);           \
   template int prepare_acoustic_reg<R>(int);              \
+  template void launch_moist_terms<R>(const Layout&, const DBase<R>&, const R*, const R*, const R*, R*, R*, \
+                                      cudaStream_t);      \
   template int launch_acoustic_column_reg<R>(const AcouArgs<R>&, const R*, int, cudaStream_t);
 WFE_INST(float)
 WFE_INST(double)

@@ -62,6 +62,7 @@ struct AcouArgs {
   R* th_out;
   const R *n_pip, *n_thp;          // time-n pi', theta' (ghost values)
   const R *qv, *qc, *qr;           // time-n moisture, stage constant
+  const R *mq, *mb;                // its terms in the column (launch_moist_terms) or null
   const R *tu, *tv, *tw, *tth, *tpi;  // tpi may be null (no slow pi' tendency)
 };
 
@@ -412,6 +413,13 @@ int prepare_acoustic_fused(int nz);
 template <typename R>
 int launch_acoustic_column_reg(const AcouArgs<R>& a, const R* prof, int s, cudaStream_t st);
 int acoustic_reg_shapes();
+// The moisture terms of the column on the inner w levels, from the time-n
+// species: mq the factor of theta_v^w, mb the moist part of the buoyancy
+// (AcouArgs::mq, mb: what the register-held kernel reads instead of the four
+// fields).
+template <typename R>
+void launch_moist_terms(const Layout& L, const DBase<R>& b, const R* qv, const R* qc, const R* qr, R* mq, R* mb,
+                        cudaStream_t st);
 template <typename R>
 bool acoustic_reg_fits(int nz, int s);
 template <typename R>
