@@ -499,3 +499,20 @@ def test_parallel_solve_column_agrees_to_rounding(name, prec, tol, monkeypatch):
             e = scaled_err(_interior(c, out["16"][k], k), _interior(o, it.field(k), k))
             c.close()
             assert e <= 1e-10, (k, e)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("nx,ny,nz", [(18, 18, 12), (61, 40, 40), (70, 41, 90)])
+def test_padded_transfers_roundtrip(nx, ny, nz, prec):
+    """A padded upload converted by one thread and by several (fields of 0.1, 1.2
+    and 2.7 MB) and its download give every point back, ghosts included."""
+    ov = {"nx": str(nx), "ny": str(ny), "nz": str(nz)}
+    c = W.Case(CASES / "bubble_open.ini", ov, precision=prec)
+    a = np.random.default_rng(nz).standard_normal(c.shape)
+    want = a if prec == "f64" else a.astype(np.float32).astype(np.float64)
+    for dtype in (np.float64, np.float32):
+        c.set_field("thp", a.astype(dtype))
+        got = c.field("thp")
+        assert np.array_equal(got, want if dtype == np.float64 else a.astype(np.float32).astype(np.float64))
+    c.close()
