@@ -470,9 +470,10 @@ __global__ void __launch_bounds__(256, kUvMinBlocks<R>) k_acoustic_uv_batch(Batc
 // gradient spelled out, so that no two levels of a thread share one):
 // bit-identical.
 //
-// What bounds it: uv_body issues about 310 instructions per 32 points, of
-// which an eighth is arithmetic; the march issues about a third of that and
-// is left waiting for its loads.  KS trades instructions against resident
+// What bounds it: the latency of its loads (5.7 of 15 cycles between a warp's
+// issues) at a quarter of DRAM's rate.  It issues 7.8 M warp instructions on
+// 160x160x40 where uv_body issues 10.0 M, an eighth of them arithmetic, and
+// has no barrier.  KS trades instructions against resident
 // threads: one level wins on flat grids, two over terrain, and uv_body's
 // blocks on grids of a few rows, where the edge points are a third of all
 // (the tuner picks; four levels a thread were slower everywhere).  Per launch

@@ -15,9 +15,10 @@
 // PROF: the coefficients that depend on the level alone from per-level tables
 // (PipeColParams::prof in kernels.cuh) instead of seven fields.
 //
-// What bounds it: the latency of each warp's own instructions (about 300 a
-// level and warp, the serial sweep behind a barrier among them), not memory:
-// DRAM is at a quarter of its rate.  So the shapes trade registers against
+// What bounds it: the barrier behind the serial sweep (9 of 19 cycles between
+// a warp's issues with two CTAs per SM) and the latency of each warp's own
+// instructions (about 260 a level), not memory: DRAM is at a fifth of its
+// rate.  So the shapes trade registers against
 // resident warps; 16 to 32 columns with three or four levels a thread win on
 // large grids, 8 columns on small ones, and the tuner picks.  Per launch
 // (event-timed inside a step, 4.7 us of event nodes included) against the
