@@ -1413,9 +1413,9 @@ class ModelT final : public Model {
   // When every column of the run-constant column coefficients (the
   // reference's rtjx, rtjy, aw, kt3, theta_b^w, dtheta_b/dz, qv_b) holds the
   // same values level by level -- flat ground and a uniform map factor --
-  // the pipelined column kernels read them from per-level tables
-  // (the values of column (0, 0)) instead of streaming a box of each per
-  // tile: the same values, bit for bit.  Checked over the points the column
+  // the register-held and the pipelined column kernels read them from
+  // per-level tables (the values of column (0, 0)) instead of seven fields:
+  // the same values, bit for bit.  Checked over the points the column
   // kernel reads.  Likewise the base state's thb, pib, rhob and rhobw for
   // the mass-flux, Kessler and u, v kernels (DBase::lvl), checked over every
   // column they read (the interior and its three-wide ring) at levels
@@ -1479,8 +1479,6 @@ class ModelT final : public Model {
     return (R*)p;
   }
 
-  // reference padded layout -> pitched; columns/rows outside the reference's
-  // padded range replicate the nearest one so that no padding is uninitialised
   // Runs f(k0, k1) over the padded levels, in a few threads when the field is
   // large: one core converts 8-byte host values at a fraction of the memory's
   // rate.  An upload of a 72 x 10 x 406 field takes 0.19 instead of 0.39 ms, of
@@ -1509,6 +1507,8 @@ class ModelT final : public Model {
     for (auto& x : th) x.join();
   }
 
+  // reference padded layout -> pitched; columns/rows outside the reference's
+  // padded range replicate the nearest one so that no padding is uninitialised
   void to_pitched(const double* ref, R* out) {
     over_levels([&](int k0, int k1) {
       const int n = g_.NX;  // row columns -3 .. nx + 2; the pitch's edges repeat them
