@@ -86,6 +86,25 @@ def test_moist_dot_product(ov, prec, tol):
     c.close()
 
 
+@pytest.mark.parametrize("prec,tol", [("f64", 1e-10), ("f32", 1e-4)])
+@pytest.mark.parametrize("nx,ny,nz", [(16, 16, 4), (16, 16, 5), (16, 16, 9), (16, 16, 18), (16, 16, 100), (24, 100, 80),
+                                      (80, 48, 16), (83, 80, 16)])
+def test_dot_product_over_the_column_kernels_shapes(nx, ny, nz, prec, tol):
+    """Sweeps with a remainder and without a full block of four and eight rows;
+    columns so deep that an SM holds one or two CTAs; grids large enough for 16
+    level lanes, bounded for four CTAs per SM (80 x 48) and, in FP64, for six
+    (83 x 80, ragged)."""
+    c = W.Case(CASES / "wk82_small.ini", overrides=dict(PERIODIC, nx=str(nx), ny=str(ny), nz=str(nz),
+                                                        dz=str(8000 // nz), stretch="none"), precision=prec)
+    x0 = A.get_fields(c)
+    rng = np.random.default_rng(nz)
+    sc = {"qv": 1e-3, "qc": 1e-3, "qr": 1e-3}
+    dx, y = _rand(c, rng, A.FIELDS8, sc), _rand(c, rng, A.FIELDS8, sc)
+    lhs, rhs = _dot(A.tangent(c, x0, dx, 2), y), _dot(dx, A.adjoint(c, x0, y, 2))
+    assert abs(lhs - rhs) <= tol * max(abs(lhs), abs(rhs)), (lhs, rhs)
+    c.close()
+
+
 def test_moist_gradient_matches_central_differences():
     c, x0 = _moist_state("f64", PERIODIC)
     n = 6

@@ -894,10 +894,9 @@ __global__ void __launch_bounds__(256, kUvLinMinBlocks<R>) k_ad_uv_cells(AcouArg
 // per column, everything else in parallel over the levels.
 // FP32 tiles hold 16 columns, FP64 8, so that the adjoint's arrays for
 // lin_max_levels() levels fit in shared memory; the level lanes beside them
-// are chosen per launch (lin_lanes)
+// are chosen per launch (lin_shape)
 template <typename R>
 constexpr int kLcx = sizeof(R) == 4 ? 16 : 8;
-constexpr int kLinColThreads = 512;
 
 // Tridiagonal sweeps over rows 1..n-1 (row 1 without the lower, row n-1
 // without the upper coefficient) in one thread, arrays strided by kLcx<R>:
@@ -962,7 +961,8 @@ __device__ __forceinline__ void eliminate(int n, Low low, const R* B, Up up, con
   }
 }
 
-// rinv: null, or where the rows' reciprocals go (not one of the inputs)
+// rinv: null, or where the rows' reciprocals go: may be B, whose rows a step
+// has read before it stores theirs (the read-ahead past the last row is unused)
 template <typename R, bool RINV = false>
 __device__ __forceinline__ void thomas_s(int n, const R* A, const R* B, const R* C, const R* D, R* cs, R* ds,
                                          R* x, R* rinv = nullptr) {
@@ -1053,10 +1053,10 @@ struct ColGeom {
 // surface w at level 0).  Ends with a barrier.
 enum { V_AV, V_SV, V_P, V_E, V_G, V_A, V_B, V_C, V_D, V_W, V_CS, V_DS, V_N };
 
-// RINV: the rows' reciprocals into array `rinv` for a second solve.
+// RINV: B ends as the rows' reciprocals, for a second solve.
 template <typename R, bool RINV = false>
 __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColGeom<R>& g, bool active,
-                                                const ColArr<R>& S, int rinv = 0) {
+                                                const ColArr<R>& S) {
   const Layout& L = a.L;
   const int nz = g.nz, tx = threadIdx.x, lane = threadIdx.y;
   const R dtau = g.dtau, c1 = g.c1, c2 = g.c2;
@@ -1127,7 +1127,7 @@ __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColG
   __syncthreads();
   if (active && lane == 0) {
     R* W = S[V_W] + tx;
-    thomas_s<R, RINV>(nz, A, B, C, D, S[V_CS] + tx, S[V_DS] + tx, W, RINV ? S[rinv] + tx : nullptr);
+    thomas_s<R, RINV>(nz, A, B, C, D, S[V_CS] + tx, S[V_DS] + tx, W, RINV ? B : nullptr);
     R us = (R)0.5 * (u[g.c0] + u[g.c0 + sx]);
     R vs = (R)0.5 * (v[g.c0] + v[g.c0 + sy]);
     W[0] = us * g.hxc + vs * g.hyc;
@@ -1186,10 +1186,10 @@ __device__ __forceinline__ void column_values_stored_s(const AcouArgs<R>& a, con
   __syncthreads();
 }
 
-enum { T_DSV = V_N, T_DTH, T_DP, T_RHS, T_DW, T_RINV, T_NARR };
+enum { T_DSV = V_N, T_DTH, T_DP, T_RHS, T_DW, T_NARR };
 
-template <typename R>
-__global__ void __launch_bounds__(kLinColThreads) k_tl_column(AcouArgs<R> a, AcouArgs<R> d, int with_forward) {
+template <typename R, int KL, int NB>
+__global__ void __launch_bounds__(kLcx<R> * KL, NB) k_tl_column(AcouArgs<R> a, AcouArgs<R> d, int with_forward) {
   extern __shared__ __align__(16) unsigned char lin_smem[];
   const Layout& L = a.L;
   const int tx = threadIdx.x, lane = threadIdx.y;
@@ -1208,7 +1208,7 @@ __global__ void __launch_bounds__(kLinColThreads) k_tl_column(AcouArgs<R> a, Aco
   if (active)
 #pragma unroll 4
     for (int k = lane; k < nz; k += (int)blockDim.y) dth[k * kLcx<R>] = d.th_in[g.at(k)];
-  column_values_s<R, true>(a, g, active, S, T_RINV);
+  column_values_s<R, true>(a, g, active, S);
   const R *Av = S[V_AV] + tx, *P = S[V_P] + tx, *E = S[V_E] + tx, *G = S[V_G] + tx;
   const R* W = S[V_W] + tx;
   if (active)
@@ -1272,7 +1272,7 @@ __global__ void __launch_bounds__(kLinColThreads) k_tl_column(AcouArgs<R> a, Aco
     }
   __syncthreads();
   if (active && lane == 0) {
-    resolve_s(nz, S[V_A] + tx, S[T_RINV] + tx, rhs, S[V_CS] + tx, S[V_DS] + tx, dw);
+    resolve_s(nz, S[V_A] + tx, S[V_B] + tx, rhs, S[V_CS] + tx, S[V_DS] + tx, dw);
     dw[0] = (R)0.5 * (du[g.c0] + du[g.c0 + sx]) * g.hxc + (R)0.5 * (dv[g.c0] + dv[g.c0 + sy]) * g.hyc;
   }
   __syncthreads();
@@ -1312,8 +1312,8 @@ enum { A_WB = V_N, A_PB, A_TB, A_WS, A_LAM, A_GL, A_PIB, A_THB, A_KTD, A_NARR };
 // to the faces.
 // STORED: the forward values from the launch's outputs (column_values_stored_s)
 // instead of recomputing the forward column
-template <typename R, bool STORED = false>
-__global__ void __launch_bounds__(kLinColThreads) k_ad_column(AcouArgs<R> a, AcouArgs<R> d, R* dhB, R* svB) {
+template <typename R, int KL, int NB, bool STORED>
+__global__ void __launch_bounds__(kLcx<R> * KL, NB) k_ad_column(AcouArgs<R> a, AcouArgs<R> d, R* dhB, R* svB) {
   extern __shared__ __align__(16) unsigned char lin_smem[];
   const Layout& L = a.L;
   const int tx = threadIdx.x, lane = threadIdx.y;
@@ -1611,15 +1611,9 @@ void ad_uv(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr,
   k_ad_uv_cells<R><<<grid_cells<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, w);
 }
 
-// Level lanes of a column CTA: 16, or 32 where the grid gives an SM at most
-// two CTAs (nothing else is resident to hide a lane's serial levels).
-// Tangent-linear run per step, FP32, 8 / 16 / 32 lanes: 400x4x65 slab (100
-// CTAs) 0.71 / 0.60 / 0.56 ms, 96x96x40 1.20 / 1.16 / 1.30, 160x160x40 3.1 /
-// 2.9 / 3.4; adjoint run of the slab 1.21 / 1.12 / 1.10.
 template <typename R>
-static int lin_lanes(const Layout& L) {
-  constexpr int kFewCtas = 2 * 148;
-  return (L.nx + kLcx<R> - 1) / kLcx<R> * L.ny <= kFewCtas ? 32 : 16;
+static dim3 lin_col_grid(const Layout& L) {
+  return dim3((L.nx + kLcx<R> - 1) / kLcx<R>, L.ny);
 }
 
 int lin_max_levels() { return 160; }  // FP64 adjoint column arrays within 227 KB
@@ -1629,44 +1623,98 @@ static size_t lin_col_smem(int nz) {
   return (size_t)NARR * (nz + 1) * kLcx<R> * sizeof(R);
 }
 
+// Shape of a column launch: level lanes, and the CTAs per SM its registers are
+// bounded for.
+//
+// 32 lanes where an SM holds at most two CTAs, by the grid or by their shared
+// memory (nothing else is resident to hide a lane's serial levels), else 16.
+// Per step, 16 / 32 lanes, tangent-linear | adjoint run: FP32 400x4x65 (100
+// CTAs) 0.64 / 0.60 | 1.15 / 1.14 ms, 96x96x40 1.14 / 1.28 | 1.86 / 1.95,
+// 100x100x75 (two CTAs by shared memory) 3.11 / 2.88 | 4.31 / 4.25; FP64
+// 32x32x60 0.71 / 0.62 | 1.32 / 1.25, 96x96x40 1.98 / 2.27 | 3.19 / 3.39,
+// 64x60x150 4.52 / 3.52 | 5.89 / 5.16, 100x100x75 4.98 / 4.72 | 7.70 / 7.63.
+//
+// The sweeps' read-ahead wants about 130 registers in FP64: bounded for four
+// 16-lane CTAs it spills nothing, for six it has 80 and spills 24-56 bytes, so
+// six are taken only where they fit and save a wave of the grid: four / six,
+// 150x90x24 1.95 / 1.79 | 3.04 / 2.90 ms, 160x150x16 2.26 / 2.08 | 3.59 / 3.42,
+// but 90x90x32 (two waves either way) 1.57 / 1.74, 900x5x33 0.865 / 0.911.
+// In FP32 four 256-thread or two 512-thread CTAs leave 64 registers, and the
+// tangent spills 12 bytes.
+struct LinShape {
+  int kl, nb;
+};
+constexpr int kLinSms = 148;  // SMs of a B200
+
+template <typename R>
+static LinShape lin_shape(const Layout& L, size_t smem) {
+  const dim3 g = lin_col_grid<R>(L);
+  const long ctas = (long)g.x * g.y;
+  const int fit = (int)(228 * 1024 / (smem + 1024));  // a CTA's own KB beside its arrays
+  if (ctas <= 2 * kLinSms || fit <= 2) return {32, 2};
+  auto waves = [&](int n) { return (ctas + n * kLinSms - 1) / (n * kLinSms); };
+  return {16, sizeof(R) == 8 && fit >= 6 && waves(6) < waves(4) ? 6 : 4};
+}
+
+// f(kernel of the shape), of the tangent (TL) or the adjoint column
+template <typename R, int KL, int NB, bool TL, bool STORED, class F>
+static void lin_kernel(F&& f) {
+  if constexpr (TL) f(k_tl_column<R, KL, NB>);
+  else f(k_ad_column<R, KL, NB, STORED>);
+}
+template <typename R, bool TL, bool STORED, class F>
+static void lin_with(LinShape s, F&& f) {
+  if (s.kl == 32) lin_kernel<R, 32, 2, TL, STORED>(f);
+  else if (sizeof(R) == 8 && s.nb == 6) lin_kernel<R, 16, sizeof(R) == 8 ? 6 : 4, TL, STORED>(f);
+  else lin_kernel<R, 16, 4, TL, STORED>(f);
+}
+
 // Sets the dynamic shared-memory limits of the column kernels for nz levels,
 // once, outside any stream capture.
 template <typename R>
 int lin_prepare(int nz) {
   if (nz > lin_max_levels()) return 2;
-  if (raise_smem_limit(k_tl_column<R>, lin_col_smem<R, T_NARR>(nz)) != cudaSuccess ||
-      raise_smem_limit(k_ad_column<R>, lin_col_smem<R, A_NARR>(nz)) != cudaSuccess ||
-      raise_smem_limit(k_ad_column<R, true>, lin_col_smem<R, A_NARR>(nz)) != cudaSuccess)
-    return 1;
-  return lin_kessler_prepare<R>(nz);
+  bool bad = false;
+  for (const LinShape s : {LinShape{32, 2}, LinShape{16, 4}, LinShape{16, 6}}) {
+    auto limit = [&](size_t sm) { return [&bad, sm](auto* k) { bad |= raise_smem_limit(k, sm) != cudaSuccess; }; };
+    lin_with<R, true, false>(s, limit(lin_col_smem<R, T_NARR>(nz)));
+    lin_with<R, false, false>(s, limit(lin_col_smem<R, A_NARR>(nz)));
+    lin_with<R, false, true>(s, limit(lin_col_smem<R, A_NARR>(nz)));
+  }
+  return bad ? 1 : lin_kessler_prepare<R>(nz);
 }
 
 template <typename R>
 int tl_column(const AcouArgs<R>& a, const AcouArgs<R>& d, bool with_forward, cudaStream_t st) {
   if (a.L.nz > lin_max_levels()) return 2;
   const size_t sm = lin_col_smem<R, T_NARR>(a.L.nz);
-  k_tl_column<R><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, lin_lanes<R>(a.L)), sm, st>>>(
-      a, d, with_forward ? 1 : 0);
+  const LinShape s = lin_shape<R>(a.L, sm);
+  lin_with<R, true, false>(s, [&](auto* k) {
+    k<<<lin_col_grid<R>(a.L), dim3(kLcx<R>, s.kl), sm, st>>>(a, d, with_forward ? 1 : 0);
+  });
+  return 0;
+}
+
+template <typename R, bool STORED>
+static int launch_ad_column(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
+  if (a.L.nz > lin_max_levels()) return 2;
+  const size_t sm = lin_col_smem<R, A_NARR>(a.L.nz);
+  const LinShape s = lin_shape<R>(a.L, sm);
+  lin_with<R, false, STORED>(s, [&](auto* k) {
+    k<<<lin_col_grid<R>(a.L), dim3(kLcx<R>, s.kl), sm, st>>>(a, d, scr.f[0], scr.f[1]);
+  });
+  k_ad_column_uv<R><<<grid_uv<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, scr.f[0], scr.f[1]);
   return 0;
 }
 
 template <typename R>
 int ad_column(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
-  if (a.L.nz > lin_max_levels()) return 2;
-  const size_t sm = lin_col_smem<R, A_NARR>(a.L.nz);
-  k_ad_column<R><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, lin_lanes<R>(a.L)), sm, st>>>(a, d, scr.f[0], scr.f[1]);
-  k_ad_column_uv<R><<<grid_uv<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, scr.f[0], scr.f[1]);
-  return 0;
+  return launch_ad_column<R, false>(a, d, scr, st);
 }
 
 template <typename R>
 int ad_column_stored(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
-  if (a.L.nz > lin_max_levels()) return 2;
-  const size_t sm = lin_col_smem<R, A_NARR>(a.L.nz);
-  k_ad_column<R, true><<<dim3((a.L.nx + kLcx<R> - 1) / kLcx<R>, a.L.ny), dim3(kLcx<R>, lin_lanes<R>(a.L)), sm, st>>>(
-      a, d, scr.f[0], scr.f[1]);
-  k_ad_column_uv<R><<<grid_uv<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, scr.f[0], scr.f[1]);
-  return 0;
+  return launch_ad_column<R, true>(a, d, scr, st);
 }
 
 #define WFE_INST(R)                                                              \
