@@ -417,6 +417,27 @@ def test_tendency_variants_bit_identical_with_limiter_and_relaxation(name, prec,
 
 
 @pytest.mark.gpu
+def test_tuned_variants_are_kept_by_terrain_and_tables(monkeypatch, tmp_path):
+    """Cases of one grid and physics on flat ground, on flat ground without the
+    per-level tables and over a hill are tuned each for itself: the kernels'
+    ranking differs, and a pick is kept on disk."""
+    cache = tmp_path / "tune.txt"
+    monkeypatch.setenv("WFE_TUNE_CACHE", str(cache))
+    keys = []
+    for terrain, tables in (("none", "1"), ("none", "0"), ("gauss", "1"), ("none", "1")):
+        monkeypatch.setenv("WFE_LEVEL_TABLES", tables)
+        c = W.Case(CASES / "ops_open.ini", {"nx": "29", "ny": "11", "terrain": terrain})
+        c.step(c.dt, 0.0)
+        var = c.variants()
+        c.close()
+        line = cache.read_text().splitlines()[-1].split()
+        keys.append(line[0])
+        if len(keys) < 4:
+            assert [int(x) for x in line[1:3]] == [var["tendencies"], var["column"]] and int(line[4]) == var["uv"]
+    assert len(cache.read_text().splitlines()) == len(set(keys)) == 3
+
+
+@pytest.mark.gpu
 def test_watchdog_absmax_begin_end_matches_blocking_call():
     """The non-blocking watchdog (two page-locked slots, read one step behind)
     returns exactly what the blocking field_absmax returns for each step."""

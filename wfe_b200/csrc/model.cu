@@ -161,6 +161,8 @@ class ModelT final : public Model {
       mp[4 + q] = mbuf + 4 * n1 + q * n2;
       if (put2d(mp[4 + q], *m2[q])) return 1;
     }
+    for (const auto* slope : {&cs.m.hx_u, &cs.m.hy_v})
+      for (double x : *slope) hills_ = hills_ || x != 0;
     dm_ = DMetric<R>{mp[0], mp[1], mp[2], mp[3], mp[4], mp[5], mp[6], mp[7],
                      mp[8], mp[9], mp[10], mp[11], (R)cs.m.zt};
     // base state
@@ -853,9 +855,12 @@ class ModelT final : public Model {
     std::string name = prop.name;
     for (char& ch : name)
       if (ch == ' ') ch = '_';
-    k << "v12|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
+    // what the variants' ranking turns on besides the grid and the physics: sloping
+    // ground (one level a u, v march is the faster on flat ground, two over
+    // terrain) and which tables the column (c) and the other kernels (l) read
+    k << "v13|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
       << dp_.moisture << "pd" << dp_.pd_moist << "b" << bdy_on_ << "d" << (dp_.diff_K > 0) << "x"
-      << (pcr_allowed() ? 0 : 1);
+      << (pcr_allowed() ? 0 : 1) << "t" << hills_ << "c" << (lvl_tab_ != nullptr) << "l" << (db_.lvl != nullptr);
     return k.str();
   }
 
@@ -1671,6 +1676,7 @@ class ModelT final : public Model {
   bool reg_ok_ = false;              // register-held column variants usable
   bool pipe_ok_ = false;             // pipelined column kernels prepared
   bool tend_tma_ok_ = false;         // TMA-staged scalar tendencies usable
+  bool hills_ = false;               // the ground slopes somewhere
   R* lvl_tab_ = nullptr;             // the column coefficients' level tables (PF_*), or null
   unsigned* tma_err_ = nullptr;      // set by a TMA tile load that timed out
   std::map<std::pair<const void*, int>, CUtensorMap> tmaps_;
