@@ -438,6 +438,26 @@ def test_tuned_variants_are_kept_by_terrain_and_tables(monkeypatch, tmp_path):
 
 
 @pytest.mark.gpu
+def test_moisture_terms_take_one_field_of_memory():
+    """A moist case holds one field more than a dry one of its grid, the second
+    of the column's moisture terms (the first lies where only the fused substep
+    keeps theta')."""
+    import torch
+
+    used = {}
+    for profile in ("constant_N", "wk82", "constant_N", "wk82"):  # the first pair warms the context up
+        before = torch.cuda.mem_get_info()[0]
+        c = W.Case(CASES / "ops_open.ini", {"nx": "152", "ny": "150", "nz": "50", "dz": "300", "stretch": "none",
+                                            "profile": profile, "wind_profile": "const", "pd_moist": "off"})
+        c.step(c.dt, 0.0)
+        c.sync()
+        used[profile] = before - torch.cuda.mem_get_info()[0]
+        c.close()
+    field = 4 * 160 * 156 * 57
+    assert used["wk82"] - used["constant_N"] < 1.6 * field, used
+
+
+@pytest.mark.gpu
 def test_watchdog_absmax_begin_end_matches_blocking_call():
     """The non-blocking watchdog (two page-locked slots, read one step behind)
     returns exactly what the blocking field_absmax returns for each step."""

@@ -203,9 +203,17 @@ class ModelT final : public Model {
     if (hp_.pd_moist)
       for (int s = 0; s < 3; ++s)
         if (!(ratio_[s] = alloc(n3))) return 1;
-    if (hp_.moisture)
-      for (R*& t : mterm_)
-        if (!(t = alloc(n3))) return 1;
+    if (hp_.moisture) {
+      // the column's moisture terms: theta' has a second buffer in the fused
+      // substep only, which takes no terms; without memory for the other one
+      // the column reads the species instead
+      mterm_[0] = TH2_;
+      mterm_[1] = alloc(n3);
+      if (!mterm_[1]) {
+        cudaGetLastError();
+        err_.clear();
+      }
+    }
     // run-constant acoustic coefficients (kernels.cu:915-927)
     for (R** p : {&rtjx_, &rtjy_, &kt3_, &aw_})
       if (!(*p = alloc(n3))) return 1;
@@ -981,7 +989,7 @@ class ModelT final : public Model {
     best = 1e30f;
     // tile shapes, the fused substep kernels (number 6 stays free); the
     // register-held ones with the moisture terms a step makes for them
-    if (dp_.moisture)
+    if (dp_.moisture && mterm_[1])
       launch_moist_terms<R>(L_, db_, N[5], N[6], N[7], mterm_[0], mterm_[1], st_);
     const int nvar = acoustic_column_shapes() + 1 + acoustic_fused_shapes() + acoustic_reg_shapes() +
                      acoustic_pcr_shapes() + acoustic_pipe_pcr_shapes();
@@ -1372,7 +1380,7 @@ class ModelT final : public Model {
   // It pays on every grid measured: with against without, per step, 16x16x16
   // 166 / 168 us, 160x160x40 669 / 680 (FP64 1230 / 1312), 181x203x53 1340 /
   // 1385, 300x200x45 over terrain 3199 / 3293.
-  bool make_moist_terms() const { return dp_.moisture && mterm_[0] && reg_usable(tune_.column_cx); }
+  bool make_moist_terms() const { return dp_.moisture && mterm_[1] && reg_usable(tune_.column_cx); }
 
   // Integrator::step (src/dynamics/integrator.cpp:71-111) as launches on st_.
   int enqueue_step(R dt) {
