@@ -232,6 +232,17 @@ def test_acoustic_variants_are_bit_identical(name, prec, monkeypatch):
             assert np.array_equal(out[0][k], out[v][k]), (v, k)
 
 
+@pytest.mark.gpu
+def test_column_variant_6_is_the_first_tile_shape(monkeypatch):
+    """Number 6 has no kernel of its own: it runs the first tile shape and is
+    reported as that."""
+    monkeypatch.setenv("WFE_COLUMN_VARIANT", "6")
+    c = W.Case(CASES / "wk82_small.ini")
+    c.step(c.dt, 0.0)
+    assert c.variants()["column"] == 0
+    c.close()
+
+
 def _surface_w_error(c):
     """largest |w - (u h_x + v h_y)| of the surface points, from the run's own u
     and v (the last substep's), over the largest |u h_x| + |v h_y|"""

@@ -911,7 +911,7 @@ class ModelT final : public Model {
 
   // WFE_COLUMN_VARIANT=<n> forces the acoustic variant (0..5 column tile
   // shapes, 6 the first of them again -- the number of a kernel that is
-  // gone --, 7..9 the fused substep kernel in three tile shapes, 10..15 the register-held
+  // gone, reported as 0 --, 7..9 the fused substep kernel in three tile shapes, 10..15 the register-held
   // column kernel in six shapes, 16..18 the parallel-solve column kernel and
   // 19..22 its pipelined form, both equal to the others up to rounding),
   // WFE_UV_VARIANT=<n> the forward u, v kernel (0
@@ -928,7 +928,7 @@ class ModelT final : public Model {
       const int v = std::atoi(cv);
       if (v >= 0 && (v <= acoustic_column_shapes() || fused_usable(v) || reg_usable(v) || pcr_usable(v) ||
                      pipe_pcr_usable(v)))
-        tune_.column_cx = v;
+        tune_.column_cx = v == acoustic_column_shapes() ? 0 : v;
     }
     const char* uvv = std::getenv("WFE_UV_VARIANT");
     if (first && uvv && *uvv) {
