@@ -866,39 +866,52 @@ class ModelT final : public Model {
     // what the variants' ranking turns on besides the grid and the physics: sloping
     // ground (one level a u, v march is the faster on flat ground, two over
     // terrain) and which tables the column (c) and the other kernels (l) read
-    k << "v13|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
+    k << "v14|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
       << dp_.moisture << "pd" << dp_.pd_moist << "b" << bdy_on_ << "d" << (dp_.diff_K > 0) << "x"
       << (pcr_allowed() ? 0 : 1) << "t" << hills_ << "c" << (lvl_tab_ != nullptr) << "l" << (db_.lvl != nullptr);
     return k.str();
   }
 
+  // Best of three replays of a graph of eight calls, as the steps replay theirs:
+  // issued one by one, a small grid's launches are timed at the rate the host
+  // makes them, much the same for every variant.  Five cases tuned four times
+  // each, launches / replays: 16x16x16 took column 12, 13 or 15 with u, v 2, 3.65
+  // to 3.81 ms per 20 steps / always column 14 with u, v 0, 3.48; the 400x4x65
+  // slab u, v 1 or 3, 8.23 to 8.35 ms per 40 steps / 2, 7.99; large grids agree.
   template <class F>
   int time_ms(F&& f, float* best) {
+    *best = 1e30f;
+    cudaGraph_t gr = nullptr;
+    cudaGraphExec_t ge = nullptr;
+    CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
+    int rc = 0;
+    for (int it = 0; it < 8 && !rc; ++it) rc = f();
+    // a variant whose launch is refused (its resources do not fit) is never
+    // the fastest
+    bool refused = cudaGetLastError() != cudaSuccess;
+    refused = cudaStreamEndCapture(st_, &gr) != cudaSuccess || refused;
+    if (!rc && !refused) refused = cudaGraphInstantiate(&ge, gr, 0) != cudaSuccess;
+    if (gr) cudaGraphDestroy(gr);
+    cudaGetLastError();
+    if (rc || refused) {
+      if (ge) cudaGraphExecDestroy(ge);
+      return rc;
+    }
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    *best = 1e30f;
-    // best of three timings of eight calls each: one call of a small grid's
-    // variant takes a few microseconds, the size of the events' own jitter
     for (int rep = 0; rep < 3; ++rep) {
       CK(cudaEventRecord(e0, st_));
-      for (int it = 0; it < 8; ++it)
-        if (f()) return 1;
-      // a variant whose launch is refused (its resources do not fit) is
-      // never the fastest
-      const bool refused = cudaGetLastError() != cudaSuccess;
+      CK(cudaGraphLaunch(ge, st_));
       CK(cudaEventRecord(e1, st_));
       CK(cudaEventSynchronize(e1));
       float ms = 0;
       CK(cudaEventElapsedTime(&ms, e0, e1));
-      if (refused) {
-        *best = 1e30f;
-        break;
-      }
       if (ms < *best) *best = ms;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    cudaGraphExecDestroy(ge);
     return 0;
   }
 
