@@ -221,18 +221,6 @@ __device__ __forceinline__ R v_interior_core_m(const AcouArgs<R>& a, int c2, int
   return vin + a.dtau * (-Phys<R>::cp * thb_f * mf * grad + tin);
 }
 
-template <typename R, typename PZ>
-__device__ __forceinline__ R u_interior_core(const AcouArgs<R>& a, int c2, int kk, R tv0, R tvx, R ps0,
-                                             R psx, R uin, R tin, PZ pz) {
-  return u_interior_core_m(a, c2, kk, u_metric(a, c2, kk), tv0, tvx, ps0, psx, uin, tin, pz);
-}
-
-template <typename R, typename PZ>
-__device__ __forceinline__ R v_interior_core(const AcouArgs<R>& a, int c2, int kk, R tv0, R tvy, R ps0,
-                                             R psy, R vin, R tin, PZ pz) {
-  return v_interior_core_m(a, c2, kk, v_metric(a, c2, kk), tv0, tvy, ps0, psy, vin, tin, pz);
-}
-
 template <typename R>
 __device__ __forceinline__ R u_interior_from_m(const AcouArgs<R>& a, int c, int c2, int kk, FaceMetric<R> g,
                                                R tv0, R tvx, R ps0, R psx, R uin, R tin) {
@@ -279,20 +267,6 @@ template <typename R>
 __device__ __forceinline__ R v_interior_val(const AcouArgs<R>& a, int c, int c2, int kk, R tv0, R tvy,
                                             R ps0, R psy) {
   return v_interior_from(a, c, c2, kk, tv0, tvy, ps0, psy, a.v_in[c], a.tv[c]);
-}
-
-// Both faces of an interior point: the cell values at (i,j), (i-1,j) and
-// (i,j-1) are loaded once for the u and the v face.
-template <typename R>
-__device__ __forceinline__ void uv_pair_interior(const AcouArgs<R>& a, int i, int j, int k) {
-  const Layout& L = a.L;
-  const int kk = L.at1(k);
-  const int c = L.ati(i, j, k), c2 = L.at2i(i, j);
-  const int sy = L.px;
-  const R tv0 = theta_v_at(a, c), tvx = theta_v_at(a, c - 1), tvy = theta_v_at(a, c - sy);
-  const R ps0 = pistar_at(a, c), psx = pistar_at(a, c - 1), psy = pistar_at(a, c - sy);
-  a.u_out[c] = u_interior_val(a, c, c2, kk, tv0, tvx, ps0, psx);
-  a.v_out[c] = v_interior_val(a, c, c2, kk, tv0, tvy, ps0, psy);
 }
 
 // u on an x face (0..nx) of a row j < ny that is not an interior point:
@@ -402,7 +376,7 @@ __device__ __forceinline__ void uv_body(const AcouArgs<R>& a, int bx, int by, in
   __syncthreads();
   if (i > L.nx || j > L.ny || k >= L.nz) return;
   if (inner) {
-    // the same values uv_pair_interior loads (kernels.cu:499-526)
+    // (kernels.cu:499-526)
     if (tx > 0) {
       tvx = s_tv[tz][ty][tx - 1];
       psx = s_ps[tz][ty][tx - 1];

@@ -2,10 +2,12 @@
 // solve of one substep, src/dynamics/kernels.cu:531-645).
 //
 // A CTA owns CX columns of one row and all their levels: thread (tx, lane)
-// holds KCH consecutive levels of column tx.  It issues every global load of
-// its levels before anything waits, so a launch pays the memory latency once
-// per resident CTA instead of once per level and phase, and each field value
-// is read once.  Only what crosses the edge between two lanes' chunks goes
+// holds KCH consecutive levels of column tx.  It issues the loads of its levels'
+// state, coefficients and moisture before anything waits, so a launch pays
+// their latency once per resident CTA instead of once per level and phase, and
+// each field value is read once.  (The slow pi' tendency of relaxed runs is read
+// behind the edge exchange, theta's and d theta_b / dz while the column is
+// swept.)  Only what crosses the edge between two lanes' chunks goes
 // through shared memory (nine values up, three down), then the tridiagonal
 // rows and the solution; the Thomas sweep is the serial one of the other
 // exact column kernels (one thread per column, one reciprocal per level) with
@@ -20,7 +22,12 @@
 // instructions (about 260 a level), not memory: DRAM is at a fifth of its
 // rate.  So the shapes trade registers against
 // resident warps; 16 to 32 columns with three or four levels a thread win on
-// large grids, 8 columns on small ones, and the tuner picks.  Per launch
+// large grids, 8 columns on small ones, and the tuner picks.  A shape has one
+// cap per precision for all its forms, and most forms spill under it (bytes
+// stored, three / four levels a thread; dry, moist from the terms, from the
+// fields).  FP32 with the level tables 0, 12, 16 / 0, 28, 52, without 8, 24,
+// 40 / 32, 48, 72, relaxed 0, 36, 44 / 28, 60, 80; FP64 in 16 columns with
+// the tables 0, 0, 8 / 8, 24, 104, without 0, 8, 40 / 24, 80, 216.  Per launch
 // (event-timed inside a step, 4.7 us of event nodes included) against the
 // best of the kernels it replaced -- contiguous level chunks in registers with
 // recomputed edges, and a producer warp's ring of bulk loads in front of the

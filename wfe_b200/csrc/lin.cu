@@ -961,15 +961,15 @@ __device__ __forceinline__ void eliminate(int n, Low low, const R* B, Up up, con
   }
 }
 
-// rinv: null, or where the rows' reciprocals go: may be B, whose rows a step
+// rinv: where the rows' reciprocals go: may be B, whose rows a step
 // has read before it stores theirs (the read-ahead past the last row is unused)
-template <typename R, bool RINV = false>
+template <typename R>
 __device__ __forceinline__ void thomas_s(int n, const R* A, const R* B, const R* C, const R* D, R* cs, R* ds,
-                                         R* x, R* rinv = nullptr) {
+                                         R* x, R* rinv) {
   constexpr int X = kLcx<R>;
   auto low = [&](int k) { return A[k * X]; };
   auto up = [&](int k) { return C[k * X]; };
-  eliminate<R, decltype(low), decltype(up), RINV>(n, low, B, up, D, cs, ds, rinv);
+  eliminate<R, decltype(low), decltype(up), true>(n, low, B, up, D, cs, ds, rinv);
   back_substitute(n, cs, ds, x);
 }
 
@@ -1053,8 +1053,8 @@ struct ColGeom {
 // surface w at level 0).  Ends with a barrier.
 enum { V_AV, V_SV, V_P, V_E, V_G, V_A, V_B, V_C, V_D, V_W, V_CS, V_DS, V_N };
 
-// RINV: B ends as the rows' reciprocals, for a second solve.
-template <typename R, bool RINV = false>
+// B ends as the rows' reciprocals, for a second solve.
+template <typename R>
 __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColGeom<R>& g, bool active,
                                                 const ColArr<R>& S) {
   const Layout& L = a.L;
@@ -1127,7 +1127,7 @@ __device__ __forceinline__ void column_values_s(const AcouArgs<R>& a, const ColG
   __syncthreads();
   if (active && lane == 0) {
     R* W = S[V_W] + tx;
-    thomas_s<R, RINV>(nz, A, B, C, D, S[V_CS] + tx, S[V_DS] + tx, W, RINV ? B : nullptr);
+    thomas_s(nz, A, B, C, D, S[V_CS] + tx, S[V_DS] + tx, W, B);
     R us = (R)0.5 * (u[g.c0] + u[g.c0 + sx]);
     R vs = (R)0.5 * (v[g.c0] + v[g.c0 + sy]);
     W[0] = us * g.hxc + vs * g.hyc;
@@ -1208,7 +1208,7 @@ __global__ void __launch_bounds__(kLcx<R> * KL, NB) k_tl_column(AcouArgs<R> a, A
   if (active)
 #pragma unroll 4
     for (int k = lane; k < nz; k += (int)blockDim.y) dth[k * kLcx<R>] = d.th_in[g.at(k)];
-  column_values_s<R, true>(a, g, active, S);
+  column_values_s(a, g, active, S);
   const R *Av = S[V_AV] + tx, *P = S[V_P] + tx, *E = S[V_E] + tx, *G = S[V_G] + tx;
   const R* W = S[V_W] + tx;
   if (active)
@@ -1309,10 +1309,9 @@ enum { A_WB = V_N, A_PB, A_TB, A_WS, A_LAM, A_GL, A_PIB, A_THB, A_KTD, A_NARR };
 // Adjoint of the column.  dhB (per cell, levels < nz) receives mc times the
 // adjoint of the horizontal divergence, svB the u, v weight of level k (the
 // surface w at level 0, Sv(k) at levels 1..nz-1); k_ad_column_uv takes both
-// to the faces.
-// STORED: the forward values from the launch's outputs (column_values_stored_s)
-// instead of recomputing the forward column
-template <typename R, int KL, int NB, bool STORED>
+// to the faces.  The forward values come from the launch's outputs
+// (column_values_stored_s).
+template <typename R, int KL, int NB>
 __global__ void __launch_bounds__(kLcx<R> * KL, NB) k_ad_column(AcouArgs<R> a, AcouArgs<R> d, R* dhB, R* svB) {
   extern __shared__ __align__(16) unsigned char lin_smem[];
   const Layout& L = a.L;
@@ -1357,10 +1356,7 @@ __global__ void __launch_bounds__(kLcx<R> * KL, NB) k_ad_column(AcouArgs<R> a, A
         tb[q] = d.th_out[c];
       }
     }
-  if (STORED)
-    column_values_stored_s(a, g, active, S);
-  else
-    column_values_s(a, g, active, S);
+  column_values_stored_s(a, g, active, S);
   const R *Av = S[V_AV] + tx, *P = S[V_P] + tx, *E = S[V_E] + tx, *G = S[V_G] + tx;
   const R* W = S[V_W] + tx;
   // adjoint of the column solution w (level 0: surface w, level nz: the lid)
@@ -1635,7 +1631,7 @@ static size_t lin_col_smem(int nz) {
 // 64x60x150 4.52 / 3.52 | 5.89 / 5.16, 100x100x75 4.98 / 4.72 | 7.70 / 7.63.
 //
 // The sweeps' read-ahead wants about 130 registers in FP64: bounded for four
-// 16-lane CTAs it spills nothing, for six it has 80 and spills 24-56 bytes, so
+// 16-lane CTAs it spills nothing, for six it has 80 and spills 24 to 48 bytes, so
 // six are taken only where they fit and save a wave of the grid: four / six,
 // 150x90x24 1.95 / 1.79 | 3.04 / 2.90 ms, 160x150x16 2.26 / 2.08 | 3.59 / 3.42,
 // but 90x90x32 (two waves either way) 1.57 / 1.74, 900x5x33 0.865 / 0.911.
@@ -1657,16 +1653,16 @@ static LinShape lin_shape(const Layout& L, size_t smem) {
 }
 
 // f(kernel of the shape), of the tangent (TL) or the adjoint column
-template <typename R, int KL, int NB, bool TL, bool STORED, class F>
+template <typename R, int KL, int NB, bool TL, class F>
 static void lin_kernel(F&& f) {
   if constexpr (TL) f(k_tl_column<R, KL, NB>);
-  else f(k_ad_column<R, KL, NB, STORED>);
+  else f(k_ad_column<R, KL, NB>);
 }
-template <typename R, bool TL, bool STORED, class F>
+template <typename R, bool TL, class F>
 static void lin_with(LinShape s, F&& f) {
-  if (s.kl == 32) lin_kernel<R, 32, 2, TL, STORED>(f);
-  else if (sizeof(R) == 8 && s.nb == 6) lin_kernel<R, 16, sizeof(R) == 8 ? 6 : 4, TL, STORED>(f);
-  else lin_kernel<R, 16, 4, TL, STORED>(f);
+  if (s.kl == 32) lin_kernel<R, 32, 2, TL>(f);
+  else if (sizeof(R) == 8 && s.nb == 6) lin_kernel<R, 16, sizeof(R) == 8 ? 6 : 4, TL>(f);
+  else lin_kernel<R, 16, 4, TL>(f);
 }
 
 // Sets the dynamic shared-memory limits of the column kernels for nz levels,
@@ -1677,9 +1673,8 @@ int lin_prepare(int nz) {
   bool bad = false;
   for (const LinShape s : {LinShape{32, 2}, LinShape{16, 4}, LinShape{16, 6}}) {
     auto limit = [&](size_t sm) { return [&bad, sm](auto* k) { bad |= raise_smem_limit(k, sm) != cudaSuccess; }; };
-    lin_with<R, true, false>(s, limit(lin_col_smem<R, T_NARR>(nz)));
-    lin_with<R, false, false>(s, limit(lin_col_smem<R, A_NARR>(nz)));
-    lin_with<R, false, true>(s, limit(lin_col_smem<R, A_NARR>(nz)));
+    lin_with<R, true>(s, limit(lin_col_smem<R, T_NARR>(nz)));
+    lin_with<R, false>(s, limit(lin_col_smem<R, A_NARR>(nz)));
   }
   return bad ? 1 : lin_kessler_prepare<R>(nz);
 }
@@ -1689,32 +1684,22 @@ int tl_column(const AcouArgs<R>& a, const AcouArgs<R>& d, bool with_forward, cud
   if (a.L.nz > lin_max_levels()) return 2;
   const size_t sm = lin_col_smem<R, T_NARR>(a.L.nz);
   const LinShape s = lin_shape<R>(a.L, sm);
-  lin_with<R, true, false>(s, [&](auto* k) {
+  lin_with<R, true>(s, [&](auto* k) {
     k<<<lin_col_grid<R>(a.L), dim3(kLcx<R>, s.kl), sm, st>>>(a, d, with_forward ? 1 : 0);
   });
   return 0;
 }
 
-template <typename R, bool STORED>
-static int launch_ad_column(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
+template <typename R>
+int ad_column_stored(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
   if (a.L.nz > lin_max_levels()) return 2;
   const size_t sm = lin_col_smem<R, A_NARR>(a.L.nz);
   const LinShape s = lin_shape<R>(a.L, sm);
-  lin_with<R, false, STORED>(s, [&](auto* k) {
+  lin_with<R, false>(s, [&](auto* k) {
     k<<<lin_col_grid<R>(a.L), dim3(kLcx<R>, s.kl), sm, st>>>(a, d, scr.f[0], scr.f[1]);
   });
   k_ad_column_uv<R><<<grid_uv<R>(a.L), dim3(32, 4, 2), 0, st>>>(a, d, scr.f[0], scr.f[1]);
   return 0;
-}
-
-template <typename R>
-int ad_column(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
-  return launch_ad_column<R, false>(a, d, scr, st);
-}
-
-template <typename R>
-int ad_column_stored(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratch<R>& scr, cudaStream_t st) {
-  return launch_ad_column<R, true>(a, d, scr, st);
 }
 
 #define WFE_INST(R)                                                              \
@@ -1725,7 +1710,6 @@ int ad_column_stored(const AcouArgs<R>& a, const AcouArgs<R>& d, const LinScratc
   template void tl_uv<R>(const AcouArgs<R>&, const AcouArgs<R>&, cudaStream_t);   \
   template void ad_uv<R>(const AcouArgs<R>&, const AcouArgs<R>&, const LinScratch<R>&, cudaStream_t); \
   template int tl_column<R>(const AcouArgs<R>&, const AcouArgs<R>&, bool, cudaStream_t); \
-  template int ad_column<R>(const AcouArgs<R>&, const AcouArgs<R>&, const LinScratch<R>&, cudaStream_t); \
   template int ad_column_stored<R>(const AcouArgs<R>&, const AcouArgs<R>&, const LinScratch<R>&, cudaStream_t); \
   template void zero_ring<R>(R*, const Layout&, cudaStream_t);                        \
   template int copy_fields<R>(const CopyJob<R>&, size_t, cudaStream_t);               \

@@ -14,12 +14,14 @@
 //      the start of every segment of `every` steps (the last segment is not
 //      run there: its replay below is its forward run).  The reverse sweep
 //      takes the segments last to first: it restores the segment's start
-//      state, replays the segment forward with one graph that saves every
-//      buffer each launch overwrites (an undo log), and walks the launches
-//      backwards with a second graph: restore the launch's outputs from the
-//      log, run its AD kernel -- except the acoustic column, whose adjoint
-//      runs first and reads the forward solution from the outputs still in
-//      place (its inputs updated in place from the log).  A step is a
+//      state, replays the segment forward with one graph that saves what the
+//      launches overwrite (an undo log, one copy launch per group: a stage's
+//      fill, fluxes and tendencies; a substep's u, v and column; Kessler), and
+//      walks the groups backwards with a second graph: a stage's AD kernels,
+//      then the restore from the log; a substep's column adjoint, which reads
+//      the forward solution from the outputs still in place (its inputs
+//      updated in place from the log), then the restore, then the u, v
+//      adjoint; Kessler's restore, then its AD kernel.  A step is a
 //      function of its time-n state alone (every other buffer is written
 //      before it is read), so restoring that state reproduces the segment.
 // Cost per step: the forward pass (all segments but the last), the replay,
@@ -308,6 +310,7 @@ class LinT final : public Lin {
     return 0;
   }
 
+  // (a column launch's adjoint is ad_column_from_outputs)
   int ad(const Rec& r) {
     switch (r.kind) {
       case K_FILL: ad_fill<R>(tr(as<FillArgs<R>>(r)), st_); break;
@@ -320,11 +323,6 @@ class LinT final : public Lin {
       case K_UV: {
         const auto& a = as<AcouArgs<R>>(r);
         ad_uv<R>(a, tr(a), scr_, st_);
-        break;
-      }
-      case K_COL: {
-        const auto& a = as<AcouArgs<R>>(r);
-        if (ad_column<R>(a, tr(a), scr_, st_)) return fail("column deeper than the linearised kernels hold");
         break;
       }
       case K_KES: {
