@@ -85,3 +85,15 @@ def test_overrides_and_text_create():
     zc = a.metric("zeta_c")[3:3 + a.nz]
     expect = np.minimum(np.maximum(zc, 0) / 1500.0, 1.0) * 35
     assert np.allclose(ub[3:3 + a.nz], expect, rtol=0, atol=1e-12)
+
+
+def test_no_clear_or_copy_on_the_default_stream():
+    """The model's streams are not ordered with the default stream.  A clear left
+    there, of a buffer just allocated, could land after the kernel that fills
+    it (the acoustic coefficients of a small case set up quickly), and a copy
+    from pageable memory return before it has arrived: every clear and copy of
+    the sources names its stream."""
+    src = ROOT / "wfe_b200" / "csrc"
+    calls = [(f.name, m.group(0)) for f in sorted(src.rglob("*")) if f.suffix in (".cu", ".cpp", ".cuh", ".hpp")
+             for m in re.finditer(r"\bcudaMem(?:set|cpy)(?:2D|3D|ToSymbol|FromSymbol)?\(", f.read_text())]
+    assert not calls, calls

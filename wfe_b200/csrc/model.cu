@@ -144,7 +144,7 @@ class ModelT final : public Model {
     tend_tma_ok_ = tensor_map_encoder() && tend_scal_tma_smem<R>() <= 227 * 1024 &&
                    prepare_tend_scal_tma<R>() == 0;
     CK(cudaMalloc(&tma_err_, sizeof(unsigned)));
-    CK(cudaMemset(tma_err_, 0, sizeof(unsigned)));
+    CK(cudaMemsetAsync(tma_err_, 0, sizeof(unsigned), st_));
     const size_t n3 = L_.n3(), n2 = L_.n2(), n1 = L_.pz;
     // metric
     R* mbuf = alloc(4 * n1 + 8 * n2);
@@ -258,7 +258,7 @@ class ModelT final : public Model {
     if (level_tables()) return 1;
     if (!(rain_ = alloc(n2))) return 1;
     CK(cudaMalloc(&clock_, CLK_N * sizeof(double)));
-    CK(cudaMemset(clock_, 0, CLK_N * sizeof(double)));
+    CK(cudaMemsetAsync(clock_, 0, CLK_N * sizeof(double), st_));
     CK(cudaMalloc(&wd_, sizeof(unsigned int)));
     CK(cudaMalloc(&mass_planes_, (size_t)g_.nz * sizeof(double)));
     CK(cudaMalloc(&mass_, sizeof(double)));
@@ -580,7 +580,7 @@ class ModelT final : public Model {
   int check_tma() {
     if (!tma_err_) return 0;
     unsigned e = 0;
-    CK(cudaMemcpy(&e, tma_err_, sizeof(e), cudaMemcpyDeviceToHost));
+    if (copy_now(&e, tma_err_, sizeof(e), cudaMemcpyDeviceToHost)) return 1;
     if (e) return fail("acoustic column: a TMA tile load timed out");
     return 0;
   }
@@ -605,7 +605,7 @@ class ModelT final : public Model {
       // per slot: the blocks' maximum and their count (left zero by every
       // launch); the result lands in mapped page-locked memory
       CK(cudaMalloc(&wd_async_, 4 * sizeof(unsigned int)));
-      CK(cudaMemset(wd_async_, 0, 4 * sizeof(unsigned int)));
+      CK(cudaMemsetAsync(wd_async_, 0, 4 * sizeof(unsigned int), st_));
       CK(cudaHostAlloc(&wd_host_, 2 * sizeof(unsigned int), cudaHostAllocMapped));
       CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&wd_host_dev_), wd_host_, 0));
       for (auto& e : wd_ev_) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1455,7 +1455,7 @@ class ModelT final : public Model {
     std::vector<R> host(L_.n3()), tab((size_t)PF_N * n1);
     for (int q = 0; q < PF_N; ++q) {
       if (q == PF_QVB && !dp_.moisture) continue;
-      CK(cudaMemcpy(host.data(), src[q], L_.n3() * sizeof(R), cudaMemcpyDeviceToHost));
+      if (copy_now(host.data(), src[q], L_.n3() * sizeof(R), cudaMemcpyDeviceToHost)) return 1;
       const int ilast = q == PF_RTJX ? nx : nx - 1, jlast = q == PF_RTJY ? ny : ny - 1;
       for (int k = 0; k < n1; ++k) {
         const R v = host[L_.at(0, 0, k)];
@@ -1467,8 +1467,7 @@ class ModelT final : public Model {
       }
     }
     if (!(lvl_tab_ = alloc(tab.size()))) return 1;
-    CK(cudaMemcpy(lvl_tab_, tab.data(), tab.size() * sizeof(R), cudaMemcpyHostToDevice));
-    return 0;
+    return copy_now(lvl_tab_, tab.data(), tab.size() * sizeof(R), cudaMemcpyHostToDevice);
   }
 
   int base_tables() {
@@ -1476,7 +1475,7 @@ class ModelT final : public Model {
     const R* src[BL_N] = {db_.thb, db_.pib, db_.rhob, db_.rhobw};
     std::vector<R> host(L_.n3()), tab((size_t)BL_N * pz);
     for (int q = 0; q < BL_N; ++q) {
-      CK(cudaMemcpy(host.data(), src[q], L_.n3() * sizeof(R), cudaMemcpyDeviceToHost));
+      if (copy_now(host.data(), src[q], L_.n3() * sizeof(R), cudaMemcpyDeviceToHost)) return 1;
       for (int k = -kOZ; k < pz - kOZ; ++k) {
         const R v = host[L_.at(0, 0, k)];
         tab[(size_t)q * pz + L_.at1(k)] = v;
@@ -1488,8 +1487,17 @@ class ModelT final : public Model {
     }
     R* d = alloc(tab.size());
     if (!d) return 1;
-    CK(cudaMemcpy(d, tab.data(), tab.size() * sizeof(R), cudaMemcpyHostToDevice));
+    if (copy_now(d, tab.data(), tab.size() * sizeof(R), cudaMemcpyHostToDevice)) return 1;
     db_.lvl = d;
+    return 0;
+  }
+
+  // A copy on the model's stream, which is not ordered with the default stream
+  // (a clear or copy left on that one could land after a kernel launched here,
+  // or before one queued here has read its target), waited for.
+  int copy_now(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+    CK(cudaMemcpyAsync(dst, src, bytes, kind, st_));
+    CK(cudaStreamSynchronize(st_));
     return 0;
   }
 
@@ -1500,7 +1508,7 @@ class ModelT final : public Model {
       fail(std::string("cudaMalloc: ") + cudaGetErrorString(e));
       return nullptr;
     }
-    cudaMemset(p, 0, n * sizeof(R));
+    cudaMemsetAsync(p, 0, n * sizeof(R), st_);
     allocs_.push_back(p);
     return (R*)p;
   }
@@ -1563,32 +1571,25 @@ class ModelT final : public Model {
   }
 
   // put3d / put2d / put1d overwrite buffers that queued steps may still read
-  // (boundary targets switched between runs, surface fields): the model's
-  // stream is drained first (the copies themselves are not stream-ordered,
-  // and an ensemble orders its members' streams after its own work)
+  // (boundary targets switched between runs, surface fields): the copies go
+  // through the model's stream, which an ensemble orders after its own work
   int put3d(R* d, const std::vector<double>& ref) {
     to_pitched(ref.data(), stage_tmp(L_.n3()));
-    CK(cudaStreamSynchronize(st_));
-    CK(cudaMemcpy(d, tmp_.data(), L_.n3() * sizeof(R), cudaMemcpyHostToDevice));
-    return 0;
+    return copy_now(d, tmp_.data(), L_.n3() * sizeof(R), cudaMemcpyHostToDevice);
   }
   int put2d(R* d, const std::vector<double>& ref2) {
-    CK(cudaStreamSynchronize(st_));
     R* o = stage_tmp(L_.n2());
     for (int j = -kOY; j < L_.py - kOY; ++j)
       for (int i = -kOX; i < L_.px - kOX; ++i) {
         int ic = i < -3 ? -3 : (i > g_.nx + 2 ? g_.nx + 2 : i);
         o[L_.at2(i, j)] = (R)ref2[g_.idx2(ic, j)];
       }
-    CK(cudaMemcpy(d, o, L_.n2() * sizeof(R), cudaMemcpyHostToDevice));
-    return 0;
+    return copy_now(d, o, L_.n2() * sizeof(R), cudaMemcpyHostToDevice);
   }
   int put1d(R* d, const std::vector<double>& v) {
-    CK(cudaStreamSynchronize(st_));
     R* o = stage_tmp(L_.pz);
     for (int q = 0; q < L_.pz; ++q) o[q] = (R)v[q];
-    CK(cudaMemcpy(d, o, L_.pz * sizeof(R), cudaMemcpyHostToDevice));
-    return 0;
+    return copy_now(d, o, L_.pz * sizeof(R), cudaMemcpyHostToDevice);
   }
   R* stage_tmp(size_t n) {
     if (tmp_.size() < n) tmp_.resize(n);
@@ -2050,7 +2051,8 @@ class EnsembleT final : public Ensemble {
     if (w.n > 0) {
       cudaError_t e = cudaMalloc(&w.d, items.size() * sizeof(int4));
       if (e == cudaSuccess)
-        e = cudaMemcpy(w.d, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(w.d, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, st_);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(st_);  // not the default stream: as ModelT::copy_now
       if (e != cudaSuccess) {
         fail(std::string("work list: ") + cudaGetErrorString(e));
         return nullptr;
