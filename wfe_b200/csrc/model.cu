@@ -866,52 +866,64 @@ class ModelT final : public Model {
     // what the variants' ranking turns on besides the grid and the physics: sloping
     // ground (one level a u, v march is the faster on flat ground, two over
     // terrain) and which tables the column (c) and the other kernels (l) read
-    k << "v14|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
+    k << "v15|" << name << "|" << g_.nx << "x" << g_.ny << "x" << g_.nz << "|" << (sizeof(R) * 8) << "|m"
       << dp_.moisture << "pd" << dp_.pd_moist << "b" << bdy_on_ << "d" << (dp_.diff_K > 0) << "x"
       << (pcr_allowed() ? 0 : 1) << "t" << hills_ << "c" << (lvl_tab_ != nullptr) << "l" << (db_.lvl != nullptr);
     return k.str();
   }
 
-  // Best of three replays of a graph of eight calls, as the steps replay theirs:
-  // issued one by one, a small grid's launches are timed at the rate the host
-  // makes them, much the same for every variant.  Five cases tuned four times
-  // each, launches / replays: 16x16x16 took column 12, 13 or 15 with u, v 2, 3.65
-  // to 3.81 ms per 20 steps / always column 14 with u, v 0, 3.48; the 400x4x65
-  // slab u, v 1 or 3, 8.23 to 8.35 ms per 40 steps / 2, 7.99; large grids agree.
+  // A variant's trial: eight calls captured in a graph and replayed, as the steps
+  // replay theirs.  Issued one by one, a small grid's launches are timed at the
+  // rate the host makes them, much the same for every variant.  Five cases tuned
+  // four times each, launches / replays: 16x16x16 took column 12, 13 or 15 with
+  // u, v 2, 3.65 to 3.81 ms per 20 steps / column 10 or 14 with u, v 0, 3.34 to
+  // 3.48; the 400x4x65 slab u, v 1 or 3, 8.23 to 8.35 ms per 40 steps / 2, 7.99;
+  // large grids agree.
+  struct Trial {
+    int v;
+    cudaGraphExec_t ge;
+    float ms;
+  };
   template <class F>
-  int time_ms(F&& f, float* best) {
-    *best = 1e30f;
+  int add_trial(std::vector<Trial>* t, int v, F&& f) {
     cudaGraph_t gr = nullptr;
     cudaGraphExec_t ge = nullptr;
     CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
     for (int it = 0; it < 8 && !rc; ++it) rc = f();
-    // a variant whose launch is refused (its resources do not fit) is never
-    // the fastest
+    // a variant whose launch is refused (its resources do not fit) has no trial
     bool refused = cudaGetLastError() != cudaSuccess;
     refused = cudaStreamEndCapture(st_, &gr) != cudaSuccess || refused;
-    if (!rc && !refused) refused = cudaGraphInstantiate(&ge, gr, 0) != cudaSuccess;
+    if (!rc && !refused && cudaGraphInstantiate(&ge, gr, 0) == cudaSuccess) t->push_back({v, ge, 1e30f});
     if (gr) cudaGraphDestroy(gr);
     cudaGetLastError();
-    if (rc || refused) {
-      if (ge) cudaGraphExecDestroy(ge);
-      return rc;
-    }
+    return rc;
+  }
+  // Runs the trials in three rounds and sets *best to the variant with the
+  // shortest one: in rounds, so that a clock that is still rising, or a moment's
+  // disturbance, weighs on all of them alike.
+  int pick(std::vector<Trial>* t, int* best) {
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    for (int rep = 0; rep < 3; ++rep) {
-      CK(cudaEventRecord(e0, st_));
-      CK(cudaGraphLaunch(ge, st_));
-      CK(cudaEventRecord(e1, st_));
-      CK(cudaEventSynchronize(e1));
-      float ms = 0;
-      CK(cudaEventElapsedTime(&ms, e0, e1));
-      if (ms < *best) *best = ms;
+    for (int rep = 0; rep < 3; ++rep)
+      for (Trial& x : *t) {
+        CK(cudaEventRecord(e0, st_));
+        CK(cudaGraphLaunch(x.ge, st_));
+        CK(cudaEventRecord(e1, st_));
+        CK(cudaEventSynchronize(e1));
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, e0, e1));
+        if (ms < x.ms) x.ms = ms;
+      }
+    float least = 1e30f;
+    for (Trial& x : *t) {
+      if (x.ms < least) least = x.ms, *best = x.v;
+      cudaGraphExecDestroy(x.ge);
     }
+    t->clear();
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaGraphExecDestroy(ge);
     return 0;
   }
 
@@ -972,34 +984,25 @@ class ModelT final : public Model {
     long saved = launches_;
     GhostJob<R> job = ghost_job(N, false);
     launch_fill_ghosts<R>(L_, job, dp_.bc_x_open, dp_.bc_y_open, st_);
-    float best = 1e30f;
+    std::vector<Trial> trials;
     // 0 fused, 1 split, 2 momentum + TMA-staged scalars, 3 fused with two
     // cells per thread
     for (int v = 0; v < 4; ++v) {
       if (v == 2 && !tend_tma_usable()) continue;
-      float ms;
       tune_.tend_variant = v;
-      if (time_ms([&] { tendencies(N, N, X, (R)dt, (R)dt / 3, false); return 0; }, &ms)) return 1;
-      if (ms < best) {
-        best = ms;
-        cached.tend_variant = v;
-      }
+      if (add_trial(&trials, v, [&] { tendencies(N, N, X, (R)dt, (R)dt / 3, false); return 0; })) return 1;
     }
-    best = 1e30f;
+    if (pick(&trials, &cached.tend_variant)) return 1;
     const int ns = hp_.acoustic_ns > 1 ? hp_.acoustic_ns : 1;
+    auto substep = [&] { return acoustic(N, X, (R)dt / (R)ns, 1, false); };
     // 0 and 2: one thread per face pair in square and slab-shaped blocks;
     // 1 and 3: short column marches
     for (int v = 0; v < kUvVariants; ++v) {
-      float ms;
       tune_.uv_variant = v;
-      if (time_ms([&] { return acoustic(N, X, (R)dt / (R)ns, 1, false); }, &ms)) return 1;
-      if (ms < best) {
-        best = ms;
-        cached.uv_variant = v;
-      }
+      if (add_trial(&trials, v, substep)) return 1;
     }
+    if (pick(&trials, &cached.uv_variant)) return 1;
     tune_.uv_variant = cached.uv_variant;
-    best = 1e30f;
     // tile shapes, the fused substep kernels (number 6 stays free); the
     // register-held ones with the moisture terms a step makes for them
     if (dp_.moisture && mterm_[1])
@@ -1013,17 +1016,13 @@ class ModelT final : public Model {
       // the parallel-solve variants agree with the others to rounding only:
       // the tuner picks them only where allowed (WFE_EXACT_COLUMN=0)
       if ((pcr_index(cx) >= 0 || pipe_pcr_index(cx) >= 0) && !pcr_allowed()) continue;
-      float ms;
       tune_.column_cx = cx;
       terms_on_ = make_moist_terms();
-      const int rc = time_ms([&] { return acoustic(N, X, (R)dt / (R)ns, 1, false); }, &ms);
+      const int rc = add_trial(&trials, cx, substep);
       terms_on_ = false;
       if (rc) return 1;
-      if (ms < best) {
-        best = ms;
-        cached.column_cx = cx;
-      }
     }
+    if (pick(&trials, &cached.column_cx)) return 1;
     launches_ = saved;
     CK(cudaStreamSynchronize(st_));
     CK(cudaGetLastError());
